@@ -233,16 +233,15 @@ static void plan(csu_ctx* x, Arena& a)
     m.nint = carve<int>(a, nc);
     m.nslot = carve<int>(a, nc);
     m.nei = carve<int>(a, c4);
-    m.wx = carve<double>(a, c4);
-    m.wy = carve<double>(a, c4);
-    m.ldx = carve<double>(a, c4);
-    m.ldy = carve<double>(a, c4);
+    m.lw = carve<double2>(a, c4);
+    m.ld = carve<double2>(a, c4);
     m.lm = carve<unsigned long long>(a, c4);
     m.les = carve<int>(a, c4);
     m.lrv = carve<unsigned long long>(a, nc);
     m.lq = carve<double2>(a, c4);
-    m.ex = carve<double>(a, c4);
-    m.ey = carve<double>(a, c4);
+    m.lk = carve<double2>(a, (size_t)3 * nc);
+    m.lim3 = carve<double>(a, nc);
+    m.em = carve<double2>(a, c4);
     m.fslot = carve<int>(a, c4);
     m.fnb = carve<int>(a, c4);
     m.omega = carve<double>(a, nc);
@@ -314,8 +313,6 @@ static void plan(csu_ctx* x, Arena& a)
     s.dQ = x->cfg.sst && x->cfg.time_scheme != CSU_TS_RK ? carve<double>(a, (size_t)6 * nc)
            : (x->cfg.sa && x->cfg.time_scheme == CSU_TS_DPLUR && x->cfg.sa_implicit_source) ? carve<double>(a, nc)
                                                                                             : nullptr;
-    s.gfix = carve<int2>(a, (size_t)nc * (nv + 1)); // at most one entry per cell and variable (and T)
-    s.gfix_n = carve<unsigned>(a, 1);
     if (!x->is_pack) {
         x->d_n2o = carve<int>(a, nc);
         x->d_stage = carve<double>(a, (size_t)nv * nc);
@@ -378,16 +375,14 @@ static int upload_mesh(csu_ctx* x)
     CK(up(m.nint, L.nint, sizeof(int) * nc));
     CK(up(m.nslot, L.nslot, sizeof(int) * nc));
     CK(up(m.nei, L.nei, sizeof(int) * c4));
-    CK(up(m.wx, L.wx, sizeof(double) * c4));
-    CK(up(m.wy, L.wy, sizeof(double) * c4));
-    CK(up(m.ldx, L.ldx, sizeof(double) * c4));
-    CK(up(m.ldy, L.ldy, sizeof(double) * c4));
+    CK(up(m.lw, L.lw, sizeof(double2) * c4));
+    CK(up(m.ld, L.ld, sizeof(double2) * c4));
     CK(up(m.lm, L.lm, sizeof(unsigned long long) * c4));
     CK(up(m.les, L.les, sizeof(int) * c4));
     CK(up(m.lrv, L.lrv, sizeof(unsigned long long) * nc));
     CK(up(m.lq, L.lq, sizeof(double2) * c4));
-    CK(up(m.ex, L.ex, sizeof(double) * c4));
-    CK(up(m.ey, L.ey, sizeof(double) * c4));
+    CK(up(m.lk, L.lk, sizeof(double2) * 3 * nc));
+    CK(up(m.em, L.em, sizeof(double2) * c4));
     CK(up(m.fslot, L.fslot, sizeof(int) * c4));
     CK(up(m.fnb, L.fnb, sizeof(int) * c4));
     CK(up(x->d_n2o, L.cell_new2old, sizeof(int) * nc));
@@ -610,6 +605,14 @@ static int max_nint(const csu_layout& L)
 
 static void plan_l2_window(csu_ctx* x);
 
+// the limiter's cell-size factors, once the mesh rows and parameters are on the device
+static int launch_lim3(csu_ctx* x)
+{
+    k_lim3<<<x->gb_c, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st, const_cast<double*>(x->mesh.lim3));
+    CK(cudaGetLastError());
+    return CSU_OK;
+}
+
 static int ctx_setup(csu_ctx* x)
 {
     int st;
@@ -650,6 +653,7 @@ static int ctx_setup(csu_ctx* x)
     if (!x->is_pack && (st = upload_mesh(x))) return st; // packs: pack_build fills the mesh rows
     x->prm = x->prms[0];
     if ((st = upload_prm(x)) || (st = reset_scalars(x, 0))) return st;
+    if (!x->is_pack && (st = launch_lim3(x))) return st;
     switch (x->cfg.stages) {
     case 1: x->rk = RK1; break;
     case 2: x->rk = RK2; break;
@@ -930,17 +934,12 @@ extern "C" int csu_get_state_rows(csu_ctx* x, double* const* U)
 template <int MODEL, bool DBG>
 static void launch_grad_lsq(csu_ctx* x)
 {
+    // a thread per cell and variable (and T)
+    const int g = x->gb_c * (BLOCK / GRAD_CELLS), t = GRAD_CELLS * (Model<MODEL>::NV + (x->prm.visc ? 1 : 0));
     switch (x->prm.lsq_exact) {
-    case 0: k_grad<MODEL, DBG, 0><<<x->gb_c, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st); break;
-    case 1: k_grad<MODEL, DBG, 1><<<x->gb_c, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st); break;
-    default:
-        // the rare components left undecided by the FP64 paths are finished by k_grad_fix: grid-stride over a
-        // list whose length only the device knows, two blocks per SM (strongly stretched cells, as beside a
-        // wall at y+ < 1, leave thousands of entries; an empty list costs one short launch)
-        k_grad<MODEL, DBG, 2><<<x->gb_c, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st);
-        k_grad_fix<MODEL><<<2 * x->sm_count, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st);
-        x->launches++;
-        break;
+    case 0: k_grad<MODEL, DBG, 0><<<g, t, 0, x->stream>>>(x->d_prm, x->mesh, x->st); break;
+    case 1: k_grad<MODEL, DBG, 1><<<g, t, 0, x->stream>>>(x->d_prm, x->mesh, x->st); break;
+    default: k_grad<MODEL, DBG, 2><<<g, t, 0, x->stream>>>(x->d_prm, x->mesh, x->st); break;
     }
 }
 
@@ -2150,7 +2149,7 @@ extern "C" int csu_pack_transfer(csu_ctx* from, int kf, csu_ctx* to, int kt)
 
 namespace {
 
-enum { SEG_CELL = 0, SEG_CELL4, SEG_FACE, SEG_BFACE };
+enum { SEG_CELL = 0, SEG_CELL3, SEG_CELL4, SEG_FACE, SEG_BFACE };
 
 struct SegArr {
     char* dev;
@@ -2173,10 +2172,9 @@ static std::vector<SegArr> seg_arrays(csu_ctx* x)
     auto P = [](const void* p) { return (char*)const_cast<void*>(p); };
     std::vector<SegArr> v = {
         {P(m.npts), 4, SEG_CELL}, {P(m.nint), 4, SEG_CELL}, {P(m.nslot), 4, SEG_CELL},
-        {P(m.nei), 4, SEG_CELL4}, {P(m.wx), 8, SEG_CELL4}, {P(m.wy), 8, SEG_CELL4},
-        {P(m.ldx), 8, SEG_CELL4}, {P(m.ldy), 8, SEG_CELL4}, {P(m.lm), 8, SEG_CELL4},
+        {P(m.nei), 4, SEG_CELL4}, {P(m.lw), 16, SEG_CELL4}, {P(m.ld), 16, SEG_CELL4}, {P(m.lm), 8, SEG_CELL4},
         {P(m.les), 4, SEG_CELL4}, {P(m.lrv), 8, SEG_CELL}, {P(m.lq), 16, SEG_CELL4},
-        {P(m.ex), 8, SEG_CELL4}, {P(m.ey), 8, SEG_CELL4}, {P(m.fslot), 4, SEG_CELL4}, {P(m.fnb), 4, SEG_CELL4},
+        {P(m.lk), 16, SEG_CELL3}, {P(m.em), 16, SEG_CELL4}, {P(m.fslot), 4, SEG_CELL4}, {P(m.fnb), 4, SEG_CELL4},
         {P(m.omega), 8, SEG_CELL}, {P(m.sxh), 8, SEG_CELL}, {P(m.syh), 8, SEG_CELL},
         {P(m.dslat), 8, SEG_CELL}, {P(m.color), 4, SEG_CELL},
         {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE}, {P(m.r0), 16, SEG_FACE},
@@ -2219,7 +2217,7 @@ static std::vector<const void*> seg_host(const csu_layout& L, std::vector<std::v
     int* rank = (int*)keep.back().data();
     local_wall_ranks(L, rank);
     std::vector<const void*> v = {
-        L.npts, L.nint, L.nslot, L.nei, L.wx, L.wy, L.ldx, L.ldy, L.lm, L.les, L.lrv, L.lq, L.ex, L.ey, L.fslot, L.fnb,
+        L.npts, L.nint, L.nslot, L.nei, L.lw, L.ld, L.lm, L.les, L.lrv, L.lq, L.lk, L.em, L.fslot, L.fnb,
         L.omega, L.sxh, L.syh, L.dslat, L.color,
         fe, pairs(L.fdsx, L.fdsy, nf), L.fds, pairs(L.r0x, L.r0y, nf), pairs(L.r1x, L.r1y, nf),
         pairs(L.fdx, L.fdy, nf), L.fdist,
@@ -2420,8 +2418,10 @@ static int seg_fill(csu_ctx* x, int k, const csu_layout* L, csu_ctx* src, int ks
             };
             switch (dst[a].kind) {
             case SEG_CELL: CK(cp(S.c0, D.c0, D.nc)); break;
+            case SEG_CELL3:
             case SEG_CELL4:
-                for (int j = 0; j < 4; j++) CK(cp((size_t)j * S.NC + S.c0, (size_t)j * D.NC + D.c0, D.nc));
+                for (int j = 0; j < (dst[a].kind == SEG_CELL3 ? 3 : 4); j++)
+                    CK(cp((size_t)j * S.NC + S.c0, (size_t)j * D.NC + D.c0, D.nc));
                 break;
             case SEG_FACE: if (D.nf) CK(cp(S.f0, D.f0, D.nf)); break;
             default: if (D.nb) CK(cp(S.b0, D.b0, D.nb)); break;
@@ -2441,8 +2441,10 @@ static int seg_fill(csu_ctx* x, int k, const csu_layout* L, csu_ctx* src, int ks
             };
             switch (dst[a].kind) {
             case SEG_CELL: CK(up(0, D.c0, D.nc)); break;
+            case SEG_CELL3:
             case SEG_CELL4:
-                for (int j = 0; j < 4; j++) CK(up((size_t)j * S.NC, (size_t)j * D.NC + D.c0, D.nc));
+                for (int j = 0; j < (dst[a].kind == SEG_CELL3 ? 3 : 4); j++)
+                    CK(up((size_t)j * S.NC, (size_t)j * D.NC + D.c0, D.nc));
                 break;
             case SEG_FACE: if (D.nf) CK(up(0, D.f0, D.nf)); break;
             default: if (D.nb) CK(up(0, D.b0, D.nb)); break;
@@ -2572,6 +2574,7 @@ static int pack_build(const char* who, const csu_prep* const* solves, int n, csu
                            cudaMemcpyHostToDevice);
         if (e != cudaSuccess) st = cuda_fail(e, "pack maps");
     }
+    if (!st) st = launch_lim3(x);
     // iteration state of the kept solves: one batched copy, their scalars in one read and one write
     if (!st && old && keep) {
         std::vector<Scalars> ho(old->nsolve), hn(n);

@@ -87,16 +87,15 @@ struct Mesh {
     const int* nint;
     const int* nslot;
     const int* nei;
-    const double* wx;
-    const double* wy;
-    const double* ex;
-    const double* ey;
-    const double* ldx;              // least squares: neighbour centre minus centroid
-    const double* ldy;
+    const double2* lw;              // [4][nc] gradient weights (LSQ 0)
+    const double2* em;              // [4][nc] edge midpoint minus centroid
+    const double2* ld;              // [4][nc] least squares: neighbour centre minus centroid
     const unsigned long long* lm;   // [4][nc] x87 significands of a, b, c, det
     const int* les;                 // [4][nc] exponent << 1 | sign
     const unsigned long long* lrv;  // reciprocal of det's significand
     const double2* lq;              // [4][nc] a, b, c and 1/det as exact (h, l) double-doubles
+    const double2* lk;              // [3][nc] a, b, c over det as (h, l) double-doubles
+    const double* lim3;             // (K sqrt(omega / omega_max))^3 of the limiter's epsilon^2 (k_lim3)
     const int* fslot;
     const int* fnb;                 // [4][nc] neighbour across interior face slot j, else -1
     const double* omega;
@@ -150,9 +149,6 @@ struct State {
     double* dbg_ghost;                        // optional: ghost primitives [bface][NP] (reference order)
     unsigned long long* lsq_x87;              // running count of gradient slots left to the integer x87 model
     double* dQ;                               // SST LU-SGS: source Jacobians [6][cell] (sst_source_jacobians)
-    int2* gfix;                               // gradient variables left to k_grad_fix: (cell, var | mask << 8)
-    unsigned* gfix_n;                         // entries in gfix (k_grad appends, k_grad_fix reads, the k_flux
-                                              // that follows empties it)
 };
 
 // ---------------------------------------------------------------- small helpers

@@ -86,12 +86,24 @@ __global__ void __launch_bounds__(BLOCK) k_prim(const Prm* __restrict__ P, const
 }
 
 // ------------------------------------------------------------------------------------------------
-// k_grad: solverUpdateGrad + the limiter loop of inter (solver.c:451-548).
+// k_grad: solverUpdateGrad + the limiter loop of inter (solver.c:451-548), one thread per cell and variable (and T in
+// viscous models); a block holds GRAD_CELLS cells.
 // DBG also records ghost primitives (boundaryCalcPrimitive) in reference order.
 // LSQ selects the least-squares arithmetic (Prm::lsq_exact): 0 precomputed FP64 weights, 1 the integer x87
 // model (ext80.cuh) for every component, 2 the FP64 x87 emulation and certified double-double solve of
-// lsqdd.cuh, with the integer model only for the rare components those cannot decide (k_grad_fix).
+// lsqdd.cuh, with the integer model only for the rare components those cannot decide.
+//
+// Bound by latency: a thread's chain of dependent FP64 operations and L2 loads. So a thread has one variable (four
+// lanes share a cell's double4 records), the certified solve keeps every x87 rounding in its bound instead of in
+// the arithmetic (lsq_decide), the two branches of the limiter are one, and the 1-3 % of components left undecided
+// are finished together, one per thread of the block. Against one thread per cell with the x87 sums emulated in
+// every component and k_grad_fix behind it: 3,049 mixed cells 36.7 -> 16.7 us, 30,000 laminar 37.9 -> 22, 160,000
+// triangles 68 -> 59, 500,000 170 -> 147, the 209,825-quad SA plate 109 -> 100 (events, launch gap included; at
+// 160,000 triangles 8 % of the measured copy bandwidth for the 50 MB it must move). Measured and dropped: the
+// undecided components where they arise (67 us; a warp has one nearly every time), in a kernel of their own
+// (137 us at 500,000, but 28 us at 3,049), on a warp of their own beside the next group's (109 us).
 // ------------------------------------------------------------------------------------------------
+constexpr int GRAD_CELLS = 32;
 
 // x87 constants a, b, c, det of cell c (solver.c:1063-1073, evaluated on the host in long double)
 __device__ __forceinline__ void lsq_consts(const Mesh& m, int nc, int c, X80* K)
@@ -105,6 +117,17 @@ __device__ __forceinline__ void lsq_consts(const Mesh& m, int nc, int c, X80* K)
     }
 }
 
+// k_lim3: the cell-size factor of limiterCalc's epsilon^2, type 0 (limiter.c:98-119), which no iteration changes.
+__global__ void __launch_bounds__(BLOCK) k_lim3(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+                                                const __grid_constant__ State s, double* lim3)
+{
+    const Prm& p = P[block_solve(s)];
+    const int c = blockIdx.x * BLOCK + threadIdx.x;
+    if (!cell_in(p, c)) return;
+    double aux = p.lim_k * sqrt(m.omega[c] / p.vol_max);
+    lim3[c] = aux * aux * aux;
+}
+
 // limiterCalc epsilon^2 of slot kk (limiter.c:98-119); aux = (K sqrt(omega / omega_max))^3 for type 0
 __device__ __forceinline__ double limiter_eps2(const Prm& p, const Scalars* sc, int kk, double aux)
 {
@@ -114,54 +137,53 @@ __device__ __forceinline__ double limiter_eps2(const Prm& p, const Scalars* sc, 
     return a2 * a2;
 }
 
-// One gradient component pair of cell c for primitive vi (T: 4) with the integer x87 model, gathering the
-// neighbours again; also the cell's value of the primitive and its range over the cell and the neighbours
-// (the limiter's inputs). Only the rare components the FP64 path cannot decide come here (k_grad_fix).
+// primitive vi (T: 4) of cell c
+__device__ __forceinline__ double cell_value(const State& s, int nc, int c, int vi)
+{
+    return vi < 4 ? reinterpret_cast<const double*>(s.W4 + c)[vi] : vi == 4 ? s.WT[c] : s.Wx[(size_t)(vi - 5) * nc + c];
+}
+
+// primitive vi (T: 4) of the neighbour (cell or ghost) in slot j of cell c
 template <int MODEL>
-__device__ __forceinline__ double2 lsq_slot_x87(const Prm& p, const Mesh& m, const State& s, int c, int vi,
-                                                double* u0p, double* qminp, double* qmaxp)
+__device__ __forceinline__ double nei_value(const Prm& p, const Mesh& m, const State& s, int c, int j, int vi)
 {
     constexpr int NP = Model<MODEL>::NP;
-    const int nc = m.nc;
-    double P0[NP];
+    const int nc = m.nc, n = m.nei[j * nc + c];
+    if (n < nc) return cell_value(s, nc, n, vi);
+    const int b = n - nc;
+    double P0[NP], Pn[NP];
     loadP<MODEL>(s, nc, c, P0);
-    double u0 = 0.0;
+    const double2 dSv = m.bn[b];
+    ghost_state<MODEL>(p, m.bflag[b], dSv.x, dSv.y, m.bds[b], P0, m.wall_d ? m.wall_d[c] : 0.0, Pn);
+    double v = Pn[0];
 #pragma unroll
-    for (int k = 0; k < NP; k++)
-        if (k == vi) u0 = P0[k];
-    *u0p = u0;
-    *qminp = u0;
-    *qmaxp = u0;
-    X80 XA = x80_zero(0), XB = x80_zero(0);
+    for (int k = 1; k < NP; k++)
+        if (k == vi) v = Pn[k];
+    return v;
+}
+
+// Gradient component (x, or y) of cell c for primitive vi with the integer x87 model, gathering the neighbours
+// again: the rare components nothing else can decide, and every component with CSU_LSQ=x87.
+template <int MODEL>
+__device__ __noinline__ double lsq_slot_x87(const Prm& p, const Mesh& m, const State& s, int c, int vi, bool y)
+{
+    const int nc = m.nc;
+    const double u0 = cell_value(s, nc, c, vi);
+    X80 X = x80_zero(0), Y = x80_zero(0);
     const int np = m.npts[c];
-    const double dw = m.wall_d ? m.wall_d[c] : 0.0;
+#pragma unroll 1
     for (int j = 0; j < np; j++) {
-        int n = m.nei[(size_t)j * nc + c];
-        double Pn[NP];
-        if (n < nc) {
-            loadP<MODEL>(s, nc, n, Pn);
-        } else {
-            int b = n - nc;
-            double2 dSv = m.bn[b];
-            ghost_state<MODEL>(p, m.bflag[b], dSv.x, dSv.y, m.bds[b], P0, dw, Pn);
-        }
-        double un = 0.0;
-#pragma unroll
-        for (int k = 0; k < NP; k++)
-            if (k == vi) un = Pn[k];
-        double du = un - u0;
-        *qmaxp = fmax(*qmaxp, un);
-        *qminp = fmin(*qminp, un);
-        XA = x80_add(XA, x80_from_double(m.ldx[(size_t)j * nc + c] * du));
-        XB = x80_add(XB, x80_from_double(m.ldy[(size_t)j * nc + c] * du));
+        const double du = nei_value<MODEL>(p, m, s, c, j, vi) - u0;
+        const double2 d = m.ld[j * nc + c];
+        X = x80_add(X, x80_from_double((y ? d.y : d.x) * du));
+        Y = x80_add(Y, x80_from_double((y ? d.x : d.y) * du));
     }
     X80 K[4];
     lsq_consts(m, nc, c, K);
-    unsigned long long rv = m.lrv[c];
-    X80 nx = x80_add(x80_mul(K[2], XA), x80_neg(x80_mul(K[1], XB)));
-    X80 ny = x80_add(x80_mul(x80_neg(K[1]), XA), x80_mul(K[0], XB));
+    // (c A - b B) / det, (-b A + a B) / det: A + B and B + A round alike
+    const X80 N = x80_add(x80_mul(y ? K[0] : K[2], X), x80_mul(x80_neg(K[1]), Y));
     atomicAdd(s.lsq_x87, 1ULL);
-    return make_double2(x80_to_double(x80_div_pre(nx, K[3], rv)), x80_to_double(x80_div_pre(ny, K[3], rv)));
+    return x80_to_double(x80_div_pre(N, K[3], m.lrv[c]));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -208,280 +230,203 @@ __global__ void __launch_bounds__(BLOCK) k_minmax(const Prm* __restrict__ P, con
     }
 }
 
-template <int MODEL, bool DBG, int LSQ>
-__global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_grad(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                                const __grid_constant__ State s)
+// The limiter of variable kk of cell c from its final gradient (limiterCalc, limiter.c:98-119), and their stores;
+// kk == NV: the temperature gradient. d1min, d1max: the variable's largest decrease and increase to a neighbour.
+template <int MODEL>
+__device__ __forceinline__ void grad_finish(const Prm& p, const Mesh& m, const State& s, const Scalars* sc, int c,
+                                            int kk, int np, double gx, double gy, double d1min, double d1max)
 {
-    constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
-    const int sid = block_solve(s);
-    const Prm& p = P[sid];
-    Scalars* const sc = s.sc + sid;
-    const int c = blockIdx.x * BLOCK + threadIdx.x;
-    if (!cell_in(p, c) || halted_behind(p, sc)) return;
-    {
-        const int nc = m.nc;
-        double P0[NP];
-        loadP<MODEL>(s, nc, c, P0);
-        double gx[NV], gy[NV], qmin[NV], qmax[NV];
-        X80 XA[NV], XB[NV], TA = x80_zero(0), TB = x80_zero(0);
-        DD AX[NV], AY[NV], TX = {0.0, 0.0}, TY = {0.0, 0.0};
-        bool sum_ok = true;
-        double gtx = 0.0, gty = 0.0;
-        const bool visc = p.visc != 0;
+    constexpr int NV = Model<MODEL>::NV;
+    const int nc = m.nc;
+    if (kk == NV) {
+        s.GTx[c] = gx;
+        s.GTy[c] = gy;
+        return;
+    }
+    double phi = 1.0;
+    if (p.order == 2) {
+        const double ee = limiter_eps2(p, sc, kk, m.lim3[c]);
 #pragma unroll
-        for (int kk = 0; kk < NV; kk++) {
-            gx[kk] = 0.0;
-            gy[kk] = 0.0;
-            qmin[kk] = P0[slot2p(kk)];
-            qmax[kk] = P0[slot2p(kk)];
-            if (LSQ == 1) {
-                XA[kk] = x80_zero(0);
-                XB[kk] = x80_zero(0);
-            }
-            if (LSQ == 2) {
-                AX[kk].h = AX[kk].l = 0.0;
-                AY[kk].h = AY[kk].l = 0.0;
-            }
-        }
-        const int np = m.npts[c];
-        const double dw = m.wall_d ? m.wall_d[c] : 0.0;
-        // the FP64 path runs the neighbour loop rolled: one copy of the gather, ghost state and x87 steps
-        constexpr int JU = LSQ == 2 ? 1 : 4;
-#pragma unroll JU
         for (int j = 0; j < 4; j++) {
-            if (j < np) {
-                int n = m.nei[(size_t)j * nc + c];
-                double Pn[NP];
-                if (n < nc) {
-                    loadP<MODEL>(s, nc, n, Pn);
-                } else {
-                    int b = n - nc;
-                    double2 dSv = m.bn[b];
-                    ghost_state<MODEL>(p, m.bflag[b], dSv.x, dSv.y, m.bds[b], P0, dw, Pn);
-                    if (DBG) {
-                        int bo = m.bold[b];
-                        for (int k = 0; k < NP; k++) s.dbg_ghost[(size_t)bo * NP + k] = Pn[k];
-                    }
-                }
-                if (LSQ != 0) {
-                    // solverCalcGrad3 (solver.c:1063-1070): double products summed in long double
-                    double dxj = m.ldx[(size_t)j * nc + c], dyj = m.ldy[(size_t)j * nc + c];
-                    if (visc) {
-                        double dT = Pn[4] - P0[4];
-                        if (LSQ == 1) {
-                            TA = x80_add(TA, x80_from_double(dxj * dT));
-                            TB = x80_add(TB, x80_from_double(dyj * dT));
-                        } else if (j == 0) {
-                            TX.h = dxj * dT;
-                            TY.h = dyj * dT;
-                        } else if (j == 1) {
-                            TX = x87_sum2(TX.h, dxj * dT, sum_ok);
-                            TY = x87_sum2(TY.h, dyj * dT, sum_ok);
-                        } else {
-                            TX = x87_sum_add(TX, dxj * dT, sum_ok);
-                            TY = x87_sum_add(TY, dyj * dT, sum_ok);
-                        }
-                    }
-#pragma unroll
-                    for (int kk = 0; kk < NV; kk++) {
-                        double du = Pn[slot2p(kk)] - P0[slot2p(kk)];
-                        if (LSQ == 1) {
-                            XA[kk] = x80_add(XA[kk], x80_from_double(dxj * du));
-                            XB[kk] = x80_add(XB[kk], x80_from_double(dyj * du));
-                        } else if (j == 0) {
-                            AX[kk].h = dxj * du;
-                            AY[kk].h = dyj * du;
-                        } else if (j == 1) {
-                            AX[kk] = x87_sum2(AX[kk].h, dxj * du, sum_ok);
-                            AY[kk] = x87_sum2(AY[kk].h, dyj * du, sum_ok);
-                        } else {
-                            AX[kk] = x87_sum_add(AX[kk], dxj * du, sum_ok);
-                            AY[kk] = x87_sum_add(AY[kk], dyj * du, sum_ok);
-                        }
-                        qmax[kk] = fmax(qmax[kk], Pn[slot2p(kk)]);
-                        qmin[kk] = fmin(qmin[kk], Pn[slot2p(kk)]);
-                    }
-                } else {
-                    double wxj = m.wx[(size_t)j * nc + c], wyj = m.wy[(size_t)j * nc + c];
-                    if (visc) {
-                        double dT = Pn[4] - P0[4];
-                        gtx += wxj * dT;
-                        gty += wyj * dT;
-                    }
-#pragma unroll
-                    for (int kk = 0; kk < NV; kk++) {
-                        double du = Pn[slot2p(kk)] - P0[slot2p(kk)];
-                        gx[kk] += wxj * du;
-                        gy[kk] += wyj * du;
-                        qmax[kk] = fmax(qmax[kk], Pn[slot2p(kk)]);
-                        qmin[kk] = fmin(qmin[kk], Pn[slot2p(kk)]);
-                    }
-                }
+            if (j < 3 || np > 3) {
+                const double2 e = m.em[j * nc + c];
+                const double d2 = (gx * e.x + gy * e.y);
+                const double phi0 = p.lim_func == 1 ? limiterBJ(d1min, d1max, d2) : limiterV2(d1min, d1max, d2, ee);
+                phi = j == 0 ? phi0 : fmin(phi, phi0);
             }
         }
-        if (LSQ != 0) {
-            // dUx = (c A - b B) / (a c - b b), dUy = (-b A + a B) / (a c - b b) in long double (solver.c:1072-1073)
-            if (LSQ == 1) {
-                X80 K[4];
-                lsq_consts(m, nc, c, K);
-                unsigned long long rv = m.lrv[c];
-#pragma unroll
-                for (int kk = 0; kk < NV; kk++) {
-                    X80 nx = x80_add(x80_mul(K[2], XA[kk]), x80_neg(x80_mul(K[1], XB[kk])));
-                    X80 ny = x80_add(x80_mul(x80_neg(K[1]), XA[kk]), x80_mul(K[0], XB[kk]));
-                    gx[kk] = x80_to_double(x80_div_pre(nx, K[3], rv));
-                    gy[kk] = x80_to_double(x80_div_pre(ny, K[3], rv));
-                }
-                if (visc) {
-                    // solverGrad_T (solver.c:477-490): the same least squares on T
-                    X80 nx = x80_add(x80_mul(K[2], TA), x80_neg(x80_mul(K[1], TB)));
-                    X80 ny = x80_add(x80_mul(x80_neg(K[1]), TA), x80_mul(K[0], TB));
-                    gtx = x80_to_double(x80_div_pre(nx, K[3], rv));
-                    gty = x80_to_double(x80_div_pre(ny, K[3], rv));
-                }
-            } else {
-                // a, b, c and 1/det as double-doubles, precomputed on the host
-                double2 qa = m.lq[c], qb = m.lq[(size_t)nc + c], qc = m.lq[(size_t)2 * nc + c];
-                double2 qr = m.lq[(size_t)3 * nc + c];
-                DD ka = {qa.x, qa.y}, kb = {qb.x, qb.y}, kc = {qc.x, qc.y}, R = {qr.x, qr.y};
-                // bit 2 kk + (0: x, 1: y) set where the cheap certified solve cannot decide; slot NV is T
-                unsigned need = 0;
-#pragma unroll
-                for (int kk = 0; kk < NV; kk++) {
-                    if (!lsq_certified(kc, kb, R, AX[kk], AY[kk], &gx[kk])) need |= 1u << (2 * kk);
-                    if (!lsq_certified(ka, kb, R, AY[kk], AX[kk], &gy[kk])) need |= 2u << (2 * kk);
-                }
-                if (visc) {
-                    if (!lsq_certified(kc, kb, R, TX, TY, &gtx)) need |= 1u << (2 * NV);
-                    if (!lsq_certified(ka, kb, R, TY, TX, &gty)) need |= 2u << (2 * NV);
-                }
-                if (!sum_ok) need = visc ? (4u << (2 * NV)) - 1u : (1u << (2 * NV)) - 1u;
-                // one out-of-loop copy of the exact-numerator solve; what that cannot decide (about one
-                // component in a thousand) is left to k_grad_fix and the integer x87 model, whose registers
-                // and code would otherwise slow every cell of this kernel
-                unsigned xneed = 0;
-#pragma unroll 1
-                while (need) {
-                    const int b = __ffs(need) - 1;
-                    need &= need - 1;
-                    const int kk = b >> 1, comp = b & 1;
-                    DD X = TX, Y = TY;
-#pragma unroll
-                    for (int q = 0; q < NV; q++) {
-                        if (q == kk) {
-                            X = AX[q];
-                            Y = AY[q];
-                        }
-                    }
-                    double g = 0.0;
-                    bool ok = sum_ok && (comp ? lsq_exact_numerator(ka, kb, R, Y, X, &g)
-                                              : lsq_exact_numerator(kc, kb, R, X, Y, &g));
-                    if (!ok) xneed |= 1u << b;
-                    if (kk == NV) {
-                        if (comp) gty = g;
-                        else gtx = g;
-                    }
-#pragma unroll
-                    for (int q = 0; q < NV; q++) {
-                        if (q == kk) {
-                            if (comp) gy[q] = g;
-                            else gx[q] = g;
-                        }
-                    }
-                }
-                // one k_grad_fix entry per (cell, variable) with undecided components
-#pragma unroll 1
-                for (int q = 0; q <= NV; q++) {
-                    const unsigned mk = (xneed >> (2 * q)) & 3u;
-                    if (mk) s.gfix[atomicAdd(s.gfix_n, 1u)] = make_int2(c, q | (int)(mk << 8));
-                }
-            }
-        }
-        if (visc) {
-            s.GTx[c] = gtx;
-            s.GTy[c] = gty;
-        }
-        double phi[NV];
-#pragma unroll
-        for (int kk = 0; kk < NV; kk++) phi[kk] = 1.0;
-        if (p.order == 2) {
-            // limiterCalc (limiter.c:98-119), type 0: eps^2 = q_inf^2 (K sqrt(omega/omega_max))^3
-            double aux = p.lim_k * sqrt(m.omega[c] / p.vol_max);
-            aux = aux * aux * aux;
-            double ee[NV];
-#pragma unroll
-            for (int kk = 0; kk < NV; kk++) ee[kk] = limiter_eps2(p, sc, kk, aux);
-#pragma unroll JU
-            for (int j = 0; j < 4; j++) {
-                if (j < np) {
-                    double exj = m.ex[(size_t)j * nc + c], eyj = m.ey[(size_t)j * nc + c];
-#pragma unroll
-                    for (int kk = 0; kk < NV; kk++) {
-                        double d2 = (gx[kk] * exj + gy[kk] * eyj);
-                        double phi0 = p.lim_func == 1 ? limiterBJ(P0[slot2p(kk)], qmin[kk], qmax[kk], d2)
-                                                      : limiterV2(P0[slot2p(kk)], qmin[kk], qmax[kk], d2, ee[kk]);
-                        phi[kk] = j == 0 ? phi0 : fmin(phi[kk], phi0);
-                    }
-                }
-            }
-        }
-        s.G4x[c] = make_double4(gx[0], gx[1], gx[2], gx[3]);
-        s.G4y[c] = make_double4(gy[0], gy[1], gy[2], gy[3]);
-        s.PH4[c] = make_double4(phi[0], phi[1], phi[2], phi[3]);
-#pragma unroll
-        for (int kk = 4; kk < NV; kk++) {
-            s.Gxx[(size_t)(kk - 4) * nc + c] = gx[kk];
-            s.Gxy[(size_t)(kk - 4) * nc + c] = gy[kk];
-            s.PHx[(size_t)(kk - 4) * nc + c] = phi[kk];
-        }
+    }
+    if (kk < 4) {
+        reinterpret_cast<double*>(s.G4x + c)[kk] = gx;
+        reinterpret_cast<double*>(s.G4y + c)[kk] = gy;
+        reinterpret_cast<double*>(s.PH4 + c)[kk] = phi;
+    } else {
+        const size_t o = (size_t)(kk - 4) * nc + c;
+        s.Gxx[o] = gx;
+        s.Gxy[o] = gy;
+        s.PHx[o] = phi;
     }
 }
 
-// ------------------------------------------------------------------------------------------------
-// k_grad_fix: the gradient components neither k_grad's certified solve nor its exact x87 numerator could
-// decide, entry (cell, variable kk (NV: temperature), mask of x / y): both components of the variable with
-// the integer x87 model (lsq_slot_x87), the undecided ones taken from it, then the variable's limiter
-// (limiterCalc) from the final gradient, as k_grad computes it. Grid-stride over the entries; k_flux, which
-// always follows, empties the list for the next gradient launch.
-// ------------------------------------------------------------------------------------------------
+// Blocks per SM of k_grad's register budget (64 registers; SST 72): with fewer the loads' latency shows (160,000
+// triangles, Euler: 4 blocks 68 us, 5 61, 6 59), with more the undecided components' code spills into the rest (8: 71).
 template <int MODEL>
-__global__ void __launch_bounds__(BLOCK) k_grad_fix(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                                    const __grid_constant__ State s)
+constexpr int grad_blocks()
 {
-    constexpr int NV = Model<MODEL>::NV;
-    const unsigned n = *s.gfix_n;
-    const int nc = m.nc;
-    for (unsigned e = blockIdx.x * BLOCK + threadIdx.x; e < n; e += gridDim.x * BLOCK) {
-        const int2 w = s.gfix[e];
-        const int c = w.x, kk = w.y & 0xff, mask = w.y >> 8;
-        const int sid = cell_solve(s, c);
-        const Prm& p = P[sid];
-        const Scalars* sc = s.sc + sid;
-        double u0, qmin, qmax;
-        const double2 gg = lsq_slot_x87<MODEL>(p, m, s, c, kk < NV ? slot2p(kk) : 4, &u0, &qmin, &qmax);
-        // the components k_grad decided are already in place
-        double* gxp = kk == NV ? s.GTx + c : kk < 4 ? reinterpret_cast<double*>(s.G4x + c) + kk
-                                                      : s.Gxx + (size_t)(kk - 4) * nc + c;
-        double* gyp = kk == NV ? s.GTy + c : kk < 4 ? reinterpret_cast<double*>(s.G4y + c) + kk
-                                                      : s.Gxy + (size_t)(kk - 4) * nc + c;
-        const double gx = (mask & 1) ? gg.x : *gxp, gy = (mask & 2) ? gg.y : *gyp;
-        *gxp = gx;
-        *gyp = gy;
-        if (kk < NV && p.order == 2) {
-            double aux = p.lim_k * sqrt(m.omega[c] / p.vol_max);
-            aux = aux * aux * aux;
-            const double ee = limiter_eps2(p, sc, kk, aux);
-            const int np = m.npts[c];
-            double phi = 1.0;
-#pragma unroll 1
-            for (int j = 0; j < np; j++) {
-                double exj = m.ex[(size_t)j * nc + c], eyj = m.ey[(size_t)j * nc + c];
-                double d2 = (gx * exj + gy * eyj);
-                double phi0 = p.lim_func == 1 ? limiterBJ(u0, qmin, qmax, d2) : limiterV2(u0, qmin, qmax, d2, ee);
-                phi = j == 0 ? phi0 : fmin(phi, phi0);
+    return MODEL == 0 ? 6 : (MODEL == 1 ? 5 : 4);
+}
+
+template <int MODEL, bool DBG, int LSQ>
+__global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), grad_blocks<MODEL>())
+    k_grad(const Prm* __restrict__ P, const __grid_constant__ Mesh m, const __grid_constant__ State s)
+{
+    constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
+    static_assert(GRAD_CELLS == 32 && BLOCK % GRAD_CELLS == 0, "blocks tile the cell blocks");
+    // undecided variables: differences, range, components; list of lane (cell of the block) | variable << 5 | mask << 8
+    __shared__ double sdu[LSQ == 2 ? NV + 1 : 1][8][GRAD_CELLS];
+    __shared__ unsigned short list[LSQ == 2 ? (NV + 1) * GRAD_CELLS : 1];
+    __shared__ unsigned nlist;
+    const int sid = s.bsolve ? s.bsolve[blockIdx.x / (BLOCK / GRAD_CELLS)] : 0;
+    const Prm& p = P[sid];
+    const Scalars* const sc = s.sc + sid;
+    // four lanes per cell for r u v p, whose records are double4; a warp each for the scalars and T
+    const int kk = threadIdx.x < 4 * GRAD_CELLS ? threadIdx.x & 3 : threadIdx.x >> 5; // variable slot; NV: T
+    const int lane = threadIdx.x < 4 * GRAD_CELLS ? threadIdx.x >> 2 : threadIdx.x & 31;
+    const int vi = kk < NV ? slot2p(kk) : 4;
+    const int c = blockIdx.x * GRAD_CELLS + lane;
+    const int nc = m.nc; // 4 nc < 2^31
+    if (LSQ == 2 && threadIdx.x == 0) nlist = 0;
+    if (LSQ == 2) __syncthreads();
+    if (cell_in(p, c) && !halted_behind(p, sc)) {
+        const double* const W = kk < 4 ? reinterpret_cast<const double*>(s.W4) + kk
+                                       : vi == 4 ? s.WT : s.Wx + (size_t)(vi - 5) * nc;
+        const int ws = kk < 4 ? 4 : 1;
+        const double u0 = W[(size_t)c * ws];
+        const int np = m.npts[c];
+        int nj[4];
+        double2 d[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (j < 3 || np > 3) {
+                nj[j] = m.nei[j * nc + c];
+                d[j] = (LSQ == 0 ? m.lw : m.ld)[j * nc + c];
             }
-            if (kk < 4) reinterpret_cast<double*>(s.PH4 + c)[kk] = phi;
-            else s.PHx[(size_t)(kk - 4) * nc + c] = phi;
+        }
+        double un[4] = {u0, u0, u0, u0};
+        unsigned ghosts = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (j < 3 || np > 3) {
+                if (nj[j] < nc) un[j] = W[(size_t)nj[j] * ws];
+                else ghosts |= 1u << j;
+            }
+        }
+        if (ghosts) {
+            double P0[NP], Pn[NP];
+            loadP<MODEL>(s, nc, c, P0);
+            const double dw = m.wall_d ? m.wall_d[c] : 0.0;
+#pragma unroll 1
+            while (ghosts) {
+                const int j = __ffs(ghosts) - 1;
+                ghosts &= ghosts - 1;
+                const int b = (j == 0 ? nj[0] : j == 1 ? nj[1] : j == 2 ? nj[2] : nj[3]) - nc;
+                double2 dSv = m.bn[b];
+                ghost_state<MODEL>(p, m.bflag[b], dSv.x, dSv.y, m.bds[b], P0, dw, Pn);
+                if (DBG && kk == 0) {
+                    int bo = m.bold[b];
+                    for (int k = 0; k < NP; k++) s.dbg_ghost[(size_t)bo * NP + k] = Pn[k];
+                }
+                double v = Pn[0];
+#pragma unroll
+                for (int k = 1; k < NP; k++)
+                    if (k == vi) v = Pn[k];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (q == j) un[q] = v;
+            }
+        }
+        double gx = 0.0, gy = 0.0, qmin = u0, qmax = u0, du[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            qmax = un[j] > qmax ? un[j] : qmax;
+            qmin = un[j] < qmin ? un[j] : qmin;
+            du[j] = un[j] - u0;
+        }
+        const double d1max = qmax - u0, d1min = qmin - u0;
+        unsigned need = 0; // bits 0 (x) and 1 (y) set where the certified solve cannot decide
+        if (LSQ == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (j < 3 || np > 3) {
+                    gx += d[j].x * du[j];
+                    gy += d[j].y * du[j];
+                }
+            }
+        } else if (LSQ == 1) {
+            gx = lsq_slot_x87<MODEL>(p, m, s, c, vi, false);
+            gy = lsq_slot_x87<MODEL>(p, m, s, c, vi, true);
+        } else {
+            // solverCalcGrad3 (solver.c:1063-1073): double products summed in long double, then
+            // dUx = (c A - b B) / (a c - b b), dUy = (-b A + a B) / (a c - b b) in long double
+            LsqSum X = lsq_sum2(d[0].x * du[0], d[1].x * du[1]), Y = lsq_sum2(d[0].y * du[0], d[1].y * du[1]);
+            lsq_sum_add(X, d[2].x * du[2]);
+            lsq_sum_add(Y, d[2].y * du[2]);
+            if (np > 3) {
+                lsq_sum_add(X, d[3].x * du[3]);
+                lsq_sum_add(Y, d[3].y * du[3]);
+            }
+            const double2 qa = m.lk[c], qb = m.lk[nc + c], qc = m.lk[2 * nc + c];
+            const DD ka = {qa.x, qa.y}, kb = {qb.x, qb.y}, kc = {qc.x, qc.y};
+            need = lsq_decide(kc, kb, X, Y, &gx) ? 0u : 1u;
+            if (!lsq_decide(ka, kb, Y, X, &gy)) need |= 2u;
+            if (need) {
+                list[atomicAdd(&nlist, 1u)] = (unsigned short)(lane | kk << 5 | need << 8);
+#pragma unroll
+                for (int j = 0; j < 4; j++) sdu[kk][j][lane] = du[j];
+                sdu[kk][4][lane] = d1min;
+                sdu[kk][5][lane] = d1max;
+                sdu[kk][6][lane] = gx;
+                sdu[kk][7][lane] = gy;
+            }
+        }
+        if (!need) grad_finish<MODEL>(p, m, s, sc, c, kk, np, gx, gy, d1min, d1max);
+    }
+    if (LSQ == 2) {
+        // The undecided variables of the whole block, one per thread: the x87 sums and the numerator exactly, and the
+        // integer model for what that cannot decide either. Done where they arise they would cost nearly every
+        // warp a pass through this code for one or two lanes.
+        __syncthreads();
+        const unsigned n = nlist;
+#pragma unroll 1
+        for (unsigned e = threadIdx.x; e < n; e += blockDim.x) {
+            const unsigned w = list[e];
+            const int l = w & 31u, q = (w >> 5) & 7u, c2 = blockIdx.x * GRAD_CELLS + l, np = m.npts[c2];
+            bool ok = true;
+            const double2 d0 = m.ld[c2], d1 = m.ld[nc + c2];
+            const double v0 = sdu[q][0][l], v1 = sdu[q][1][l];
+            DD X = x87_sum2(d0.x * v0, d1.x * v1, ok), Y = x87_sum2(d0.y * v0, d1.y * v1, ok);
+#pragma unroll 1
+            for (int j = 2; j < np; j++) {
+                const double2 dj = m.ld[j * nc + c2];
+                const double v = sdu[q][j][l];
+                X = x87_sum_add(X, dj.x * v, ok);
+                Y = x87_sum_add(Y, dj.y * v, ok);
+            }
+            const double2 qb = m.lq[nc + c2], qr = m.lq[3 * nc + c2];
+            const DD kb = {qb.x, qb.y}, R = {qr.x, qr.y};
+            double gx = sdu[q][6][l], gy = sdu[q][7][l];
+#pragma unroll 1
+            for (unsigned nd = w >> 8; nd; nd &= nd - 1) {
+                const bool y = (nd & 1u) == 0;
+                const double2 qk = m.lq[(y ? 0 : 2) * nc + c2];
+                const DD k1 = {qk.x, qk.y};
+                double g = 0.0;
+                if (!ok || !lsq_exact_numerator(k1, kb, R, y ? Y : X, y ? X : Y, &g))
+                    g = lsq_slot_x87<MODEL>(p, m, s, c2, q < NV ? slot2p(q) : 4, y);
+                if (y) gy = g;
+                else gx = g;
+            }
+            grad_finish<MODEL>(p, m, s, sc, c2, q, np, gx, gy, sdu[q][4][l], sdu[q][5][l]);
         }
     }
 }
@@ -723,8 +668,6 @@ __global__ void __launch_bounds__(FB) k_flux(const Prm* __restrict__ P, const __
                                              const __grid_constant__ State s, int nbi, const int* wall_rank,
                                              int coef)
 {
-    // k_grad_fix (always launched just before) has read its list: empty it for the next gradient launch
-    if (blockIdx.x == 0 && threadIdx.x == 0 && s.gfix_n) *s.gfix_n = 0;
     if ((int)blockIdx.x < nbi) {
         int f = blockIdx.x * FB + threadIdx.x;
         if (f >= m.nf) return;
@@ -757,8 +700,6 @@ __global__ void __launch_bounds__(FB) k_flux_st(const Prm* __restrict__ P, const
                                                 const __grid_constant__ State s, int nbi, const int* wall_rank,
                                                 int coef)
 {
-    // k_grad_fix (always launched just before) has read its list: empty it for the next gradient launch
-    if (blockIdx.x == 0 && threadIdx.x == 0 && s.gfix_n) *s.gfix_n = 0;
     if ((int)blockIdx.x >= nbi) {
         const int b = (blockIdx.x - nbi) * FB + threadIdx.x;
         if (b < m.nb) boundary_face<MODEL>(P, m, s, b, wall_rank, coef);

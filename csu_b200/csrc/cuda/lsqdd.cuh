@@ -307,4 +307,55 @@ X80_HD bool lsq_exact_numerator(DD k1, DD k2, DD R, DD X, DD Y, double* out)
     return true;
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// The same decision without the intermediate 64-bit roundings, for the gradient kernel's every component: the
+// sums A = sum_j p_j exactly (as unevaluated h + l) instead of as x87 rounds them, the solve with the constants
+// already divided by the determinant, and every x87 rounding in the bound instead of in the arithmetic. About a
+// third of the operations of x87_sum_add and lsq_certified; undecided about as often (1 to 2 components in 100).
+// ---------------------------------------------------------------------------------------------------------
+
+// Sum of products in the reference's order: h + l is the exact sum to 2^-104 b, b the sum of the |partial sums|,
+// each of which x87 rounds with relative error u = 2^-64. b == 0: every partial sum is exactly zero, in x87 too.
+struct LsqSum {
+    double h, l, b;
+};
+
+X80_HD LsqSum lsq_sum2(double p0, double p1)
+{
+    DD t = dd_two_sum(p0, p1);
+    LsqSum s = {t.h, t.l, fabs(t.h)};
+    return s;
+}
+
+X80_HD void lsq_sum_add(LsqSum& s, double p)
+{
+    DD t = dd_two_sum(s.h, p);
+    s.h = t.h;
+    s.l += t.l;
+    s.b += fabs(t.h);
+}
+
+// RN53 of the x87 value of (k1 A - k2 B) / det from the quotients k1 / det, k2 / det as double-doubles (relative
+// error <= 2^-101) when that rounding is certain. The x87 value lies within
+//     u (|k1/det| b_A + |k2/det| b_B + |k1 A/det| + |k2 B/det| + |N/det| + |q|)
+// of the exact quotient (the sums' roundings, two products, the difference, the division); the factor 1 + 2^-20
+// covers the second-order terms and this evaluation's own error (below 2^-98 of the same terms). With q = h + r,
+// |r| <= ulp(h)/2, both ends of [h + r - E, h + r + E] rounding to h puts the x87 value strictly inside h's
+// rounding interval (Ziv's test). Exactly zero in x87 when each term has a zero factor (det > 0, sums never -0).
+X80_HD bool lsq_decide(DD k1, DD k2, const LsqSum& A, const LsqSum& B, double* out)
+{
+    double p1 = k1.h * A.h, p2 = k2.h * B.h;
+    double e1 = fma(k1.l, A.h, fma(k1.h, A.l, fma(k1.h, A.h, -p1)));
+    double e2 = fma(k2.l, B.h, fma(k2.h, B.l, fma(k2.h, B.h, -p2)));
+    DD s = dd_two_sum(p1, -p2);
+    DD q = dd_two_sum(s.h, s.l + (e1 - e2));
+    double t = (fabs(p1) + fabs(p2)) + 2.0 * fabs(q.h);
+    t = fma(fabs(k1.h), A.b, t);
+    t = fma(fabs(k2.h), B.b, t);
+    double E = t * (0x1p-64 * (1.0 + 0x1p-20));
+    bool zero = (A.b == 0.0 || k1.h == 0.0) && (B.b == 0.0 || k2.h == 0.0);
+    *out = zero ? 0.0 : q.h;
+    return zero || (q.h + (q.l + E) == q.h && q.h + (q.l - E) == q.h && fabs(q.h) >= 0x1p-960 && fabs(q.h) <= 0x1p+960);
+}
+
 } // namespace csu

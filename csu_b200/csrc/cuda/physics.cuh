@@ -141,24 +141,17 @@ __device__ __forceinline__ void rotation(double* U, double dSx, double dSy, doub
     U[1] = aux;
 }
 
-// limiterV2 (limiter.c:121-147): Venkatakrishnan-type limiter of one cell edge
-__device__ __forceinline__ double limiterV2(double Ui, double Umin, double Umax, double d2, double ee)
+// limiterV2 (limiter.c:121-147): Venkatakrishnan-type limiter of one cell edge, from the largest decrease and
+// increase to a neighbour and the edge's reconstructed change. The reference's two branches share one formula,
+// evaluated once here (as branches a warp ran both); the divisor 1 of a zero change keeps its unused quotient finite.
+__device__ __forceinline__ double limiterV2(double d1min, double d1max, double d2, double ee)
 {
-    double ans;
-    double d1max = Umax - Ui;
-    double d1min = Umin - Ui;
-    if (d2 == 0) {
-        ans = 1;
-    } else if (d2 > 0) {
-        ans = (d1max * d1max + ee) * d2 + 2 * d2 * d2 * d1max;
-        ans /= d1max * d1max + 2 * d2 * d2 + d1max * d2 + ee;
-        ans /= d2;
-    } else {
-        ans = (d1min * d1min + ee) * d2 + 2 * d2 * d2 * d1min;
-        ans /= d1min * d1min + 2 * d2 * d2 + d1min * d2 + ee;
-        ans /= d2;
-    }
-    return ans;
+    const double d1 = d2 > 0 ? d1max : d1min;
+    const double dv = d2 == 0 ? 1.0 : d2;
+    double ans = (d1 * d1 + ee) * dv + 2 * dv * dv * d1;
+    ans /= d1 * d1 + 2 * dv * dv + d1 * dv + ee;
+    ans /= dv;
+    return d2 == 0 ? 1.0 : ans;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -493,11 +486,10 @@ __device__ __forceinline__ void bcInlet(const Gas& g, const double* Pa, const do
 // limiterBJ (solver.c:1132-1150): Barth-Jespersen, min(1, (Umax - Ui) / d2) -- the minmod limiter function
 // min(1, r) of the ratio of the largest admissible change to the reconstructed one. The reference defines
 // it but never calls it; here it is selected by the limiterFunc extension.
-__host__ __device__ __forceinline__ double limiterBJ(double Ui, double Umin, double Umax, double d2)
+__device__ __forceinline__ double limiterBJ(double d1min, double d1max, double d2)
 {
-    if (d2 == 0) return 1.0;
-    if (d2 > 0) return fmin(1.0, (Umax - Ui) / d2);
-    return fmin(1.0, (Umin - Ui) / d2);
+    const double q = fmin(1.0, (d2 > 0 ? d1max : d1min) / (d2 == 0 ? 1.0 : d2));
+    return d2 == 0 ? 1.0 : q;
 }
 
 // boundaryOutlet (boundary.c:53-83)

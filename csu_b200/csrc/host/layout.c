@@ -111,10 +111,10 @@ static int cmp_keyed(const void* a, const void* b)
 void csu_layout_free(csu_layout* L)
 {
     void* ptrs[] = {L->cell_new2old, L->cell_old2new, L->face_new2old, L->face_old2new, L->bface_new2old,
-                    L->bface_old2new, L->npts, L->nint, L->nslot, L->nei, L->wx, L->wy, L->ex, L->ey,
+                    L->bface_old2new, L->npts, L->nint, L->nslot, L->nei, L->lw, L->em,
                     L->fslot, L->fnb, L->omega, L->sxh, L->syh, L->xc, L->yc, L->wall_d, L->dslat, L->fe0, L->fe1,
                     L->fdsx, L->fdsy, L->fds, L->r0x, L->r0y, L->r1x, L->r1y, L->fdist, L->bown, L->bflag,
-                    L->bold, L->bdsx, L->bdsy, L->bds, L->bmx, L->bmy, L->ldx, L->ldy, L->lm, L->les, L->lrv, L->lq,
+                    L->bold, L->bdsx, L->bdsy, L->bds, L->bmx, L->bmy, L->ld, L->lm, L->les, L->lrv, L->lq, L->lk,
                     L->fdx, L->fdy, L->bdx, L->bdy, L->bL, L->bunx, L->buny, L->bds2, L->color,
                     L->color_start, L->color_cells};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) free(ptrs[i]);
@@ -157,8 +157,9 @@ int csu_layout_build(const csu_mesh_desc* m, int axi, csu_layout* L)
     ALLOC(L->face_new2old, nf); ALLOC(L->face_old2new, nf);
     ALLOC(L->bface_new2old, nb); ALLOC(L->bface_old2new, nb);
     ALLOC(L->npts, nc); ALLOC(L->nint, nc); ALLOC(L->nslot, nc); ALLOC(L->nei, c4);
-    ALLOC(L->wx, c4); ALLOC(L->wy, c4); ALLOC(L->ex, c4); ALLOC(L->ey, c4); ALLOC(L->fslot, c4); ALLOC(L->fnb, c4);
-    ALLOC(L->ldx, c4); ALLOC(L->ldy, c4); ALLOC(L->lm, c4); ALLOC(L->les, c4); ALLOC(L->lrv, nc); ALLOC(L->lq, 2 * c4);
+    ALLOC(L->lw, 2 * c4); ALLOC(L->em, 2 * c4); ALLOC(L->fslot, c4); ALLOC(L->fnb, c4);
+    ALLOC(L->ld, 2 * c4); ALLOC(L->lm, c4); ALLOC(L->les, c4); ALLOC(L->lrv, nc); ALLOC(L->lq, 2 * c4);
+    ALLOC(L->lk, (size_t)6 * nc);
     ALLOC(L->omega, nc); ALLOC(L->sxh, nc); ALLOC(L->syh, nc); ALLOC(L->xc, nc); ALLOC(L->yc, nc);
     ALLOC(L->dslat, nc);
     if (m->wall_dist) ALLOC(L->wall_d, nc);
@@ -316,8 +317,8 @@ int csu_layout_build(const csu_mesh_desc* m, int axi, csu_layout* L)
             sym += fabs(dSy);
             double xm = (m->xy[2 * p0] + m->xy[2 * p1]) * 0.5;
             double ym = (m->xy[2 * p0 + 1] + m->xy[2 * p1 + 1]) * 0.5;
-            L->ex[(size_t)j * nc + c] = xm - cx[o];
-            L->ey[(size_t)j * nc + c] = ym - cy[o];
+            L->em[2 * ((size_t)j * nc + c)] = xm - cx[o];
+            L->em[2 * ((size_t)j * nc + c) + 1] = ym - cy[o];
         }
         L->sxh[c] = sxm * 0.5;
         L->syh[c] = sym * 0.5;
@@ -361,15 +362,25 @@ int csu_layout_build(const csu_mesh_desc* m, int axi, csu_layout* L)
             double r = 1.0 / dh;
             double e = fma(-dh, r, 1.0);
             e = e - dl * r;
-            double re = e * r, rs = r + re;
+            double re = e * r, rs = r + re, rl = re - (rs - r);
             L->lq[2 * ((size_t)3 * nc + c)] = rs;
-            L->lq[2 * ((size_t)3 * nc + c) + 1] = re - (rs - r);
+            L->lq[2 * ((size_t)3 * nc + c) + 1] = rl;
+            /* a, b, c over det: double-double products with that reciprocal (2^-101 relative) */
+            for (int q = 0; q < 3; q++) {
+                double h = L->lq[2 * ((size_t)q * nc + c)], l = L->lq[2 * ((size_t)q * nc + c) + 1];
+                double p = h * rs;
+                double t = fma(h, rs, -p) + (h * rl + l * rs);
+                double z = p + t;
+                L->lk[2 * ((size_t)q * nc + c)] = z;
+                L->lk[2 * ((size_t)q * nc + c) + 1] = t - (z - p);
+            }
         }
         for (int j = 0; j < np; j++) {
-            L->ldx[(size_t)j * nc + c] = dx[j];
-            L->ldy[(size_t)j * nc + c] = dy[j];
-            L->wx[(size_t)j * nc + c] = (double)((cc * dx[j] - bb * dy[j]) / det);
-            L->wy[(size_t)j * nc + c] = (double)((-bb * dx[j] + a * dy[j]) / det);
+            size_t k2 = 2 * ((size_t)j * nc + c);
+            L->ld[k2] = dx[j];
+            L->ld[k2 + 1] = dy[j];
+            L->lw[k2] = (double)((cc * dx[j] - bb * dy[j]) / det);
+            L->lw[k2 + 1] = (double)((-bb * dx[j] + a * dy[j]) / det);
         }
 
         /* face slots: interior faces in ELEMENT.f order, then this cell's boundary faces in reference order */
@@ -470,8 +481,8 @@ int csu_layout_green_gauss(csu_layout* L)
                 }
             }
             if (!found) return CSU_ERR_INPUT;
-            L->wx[(size_t)j * nc + c] = sx * w;
-            L->wy[(size_t)j * nc + c] = sy * w;
+            L->lw[2 * ((size_t)j * nc + c)] = sx * w;
+            L->lw[2 * ((size_t)j * nc + c) + 1] = sy * w;
         }
     }
     return CSU_OK;

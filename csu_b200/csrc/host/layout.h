@@ -28,16 +28,14 @@ typedef struct csu_layout {
     int* nint;     /* interior faces                                                                  */
     int* nslot;    /* face slots = interior + boundary faces of the cell                              */
     int* nei;      /* [4][nc] neighbour (ELEMENT.neiL order): cell id, or nc + boundary face id       */
-    double* wx;    /* [4][nc] least-squares weights: dUx = sum wx (u_nei - u_cell)                     */
-    double* wy;
-    double* ldx;   /* [4][nc] neighbour centre minus centroid, x and y (solverCalcGrad3 x[jj] - x[0])   */
-    double* ldy;
+    double* lw;    /* [4][nc][2] least-squares weights: dUx = sum wx (u_nei - u_cell), dUy with wy       */
+    double* ld;    /* [4][nc][2] neighbour centre minus centroid (solverCalcGrad3 x[jj] - x[0])          */
     unsigned long long* lm;  /* [4][nc] x87 significands of a, b, c, a*c - b*b (long double, solver.c:1058-1073) */
     int* les;      /* [4][nc] exponent << 1 | sign of the same                                          */
     unsigned long long* lrv; /* [nc] invariant-divisor reciprocal of the determinant's significand       */
     double* lq;    /* [4][nc][2] a, b, c, 1/(a*c - b*b) as (high, low) double pairs                          */
-    double* ex;    /* [4][nc] edge midpoint minus centroid, edges in node order (limiter, inter)        */
-    double* ey;
+    double* lk;    /* [3][nc][2] a, b, c over (a*c - b*b) as (high, low) double pairs                        */
+    double* em;    /* [4][nc][2] edge midpoint minus centroid, edges in node order (limiter, inter)     */
     int* fslot;    /* [4][nc] +-(flux index + 1): interior faces (ELEMENT.f order) then boundary faces  */
     int* fnb;      /* [4][nc] the neighbour cell across interior face slot j (j < nint), else -1          */
     double* omega;
