@@ -222,6 +222,11 @@ static T* carve(Arena& a, size_t count)
     return p;
 }
 
+static int block_entries(int model)
+{
+    return model == 0 ? BLOCK_NE<0> : (model == 1 ? BLOCK_NE<1> : BLOCK_NE<2>);
+}
+
 // Lays out every device array of a context in one allocation (first pass sizes, second pass carves).
 static void plan(csu_ctx* x, Arena& a)
 {
@@ -298,8 +303,10 @@ static void plan(csu_ctx* x, Arena& a)
         s.Xx[k] = implicit ? carve<double>(a, (size_t)nx * nc) : nullptr;
     }
     bool dplur = x->cfg.time_scheme == CSU_TS_DPLUR;
-    s.blocks = dplur && !x->cfg.implicit_fp32 ? carve<double>(a, c4 * nv * nv) : nullptr;
-    s.blocks32 = dplur && x->cfg.implicit_fp32 ? carve<float>(a, c4 * nv * nv) : nullptr;
+    s.diag = dplur ? carve<double>(a, nc) : nullptr;
+    const size_t nblocks = (size_t)(nc + 31) / 32 * 128 * block_entries(x->model);
+    s.blocks = dplur && !x->cfg.implicit_fp32 ? carve<double>(a, nblocks) : nullptr;
+    s.blocks32 = dplur && x->cfg.implicit_fp32 ? carve<float>(a, nblocks) : nullptr;
     // partial norms: one row per 256-cell block, or per 128-cell block from the DPLUR first sweep
     s.part = carve<double>(a, (size_t)((nc + BLOCK - 1) / BLOCK) * (BLOCK / 32) * nv);
     s.bcoef = carve<double>(a, (size_t)4 * (nb > 0 ? nb : 1));
@@ -1026,7 +1033,7 @@ static void launch_blocks(csu_ctx* x)
         k_face_mit<<<(x->L.nf + BLOCK - 1) / BLOCK, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st);
         x->launches++;
     }
-    k_blocks<MODEL><<<x->max_ni * x->gb_c, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st, x->gb_c);
+    k_blocks<MODEL><<<x->max_ni * x->gb_c, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st, x->gb_c, x->max_ni);
     x->launches++;
     if (x->timing) tmark(x, KBLK);
     if (x->fin_pending) {
@@ -1049,12 +1056,12 @@ static void launch_sweep_sb(csu_ctx* x, int m, int n)
         auto* k = x->cfg.implicit_fp32
                       ? (m == n - 1 ? k_sweep<MODEL, true, true, SB, true> : k_sweep<MODEL, false, true, SB, true>)
                       : (m == n - 1 ? k_sweep<MODEL, true, true, SB, false> : k_sweep<MODEL, false, true, SB, false>);
-        k<<<x->gb_c * (BLOCK / SB), SB, 0, x->stream>>>(x->d_prm, x->mesh, x->st, m, x->xcur);
+        k<<<x->gb_c * (BLOCK / SB), SB, 0, x->stream>>>(x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
     } else {
         auto* k = x->cfg.implicit_fp32
                       ? (m == n - 1 ? k_sweep<MODEL, true, false, SB, true> : k_sweep<MODEL, false, false, SB, true>)
                       : (m == n - 1 ? k_sweep<MODEL, true, false, SB, false> : k_sweep<MODEL, false, false, SB, false>);
-        k<<<x->gb_c * (BLOCK / SB), SB, 0, x->stream>>>(x->d_prm, x->mesh, x->st, m, x->xcur);
+        k<<<x->gb_c * (BLOCK / SB), SB, 0, x->stream>>>(x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
     }
 }
 
@@ -1241,7 +1248,8 @@ static void plan_l2_window(csu_ctx* x)
     if (env && strcmp(env, "0") == 0) return;
     void* base = x->st.blocks32 ? (void*)x->st.blocks32 : (void*)x->st.blocks;
     if (!base || x->cfg.time_scheme != CSU_TS_DPLUR) return;
-    const size_t bytes = (size_t)x->max_ni * x->nv * x->nv * x->L.nc * (x->st.blocks32 ? sizeof(float) : sizeof(double));
+    const size_t bytes = (size_t)(x->L.nc + 31) / 32 * 32 * x->max_ni * block_entries(x->model) *
+                         (x->st.blocks32 ? sizeof(float) : sizeof(double));
     int max_persist = 0, max_window = 0;
     if (cudaDeviceGetAttribute(&max_persist, cudaDevAttrMaxPersistingL2CacheSize, x->device) != cudaSuccess ||
         cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, x->device) != cudaSuccess ||
@@ -1362,15 +1370,15 @@ static int time_sweep_shape(csu_ctx* x, int sb, int reps, cudaEvent_t e0, cudaEv
         switch (sb) {
         case 64:
             (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 64, true> : k_sweep<MODEL, false, false, 64, false>)
-                <<<x->gb_c * (BLOCK / 64), 64, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur);
+                <<<x->gb_c * (BLOCK / 64), 64, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
             break;
         case 256:
             (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 256, true> : k_sweep<MODEL, false, false, 256, false>)
-                <<<x->gb_c, 256, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur);
+                <<<x->gb_c, 256, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
             break;
         default:
             (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 128, true> : k_sweep<MODEL, false, false, 128, false>)
-                <<<x->gb_c * 2, 128, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur);
+                <<<x->gb_c * 2, 128, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
             break;
         }
     };
@@ -1840,18 +1848,28 @@ extern "C" int csu_dump(csu_ctx* x, int what, double* out)
             csu_set_error("csu_dump: no DPLUR blocks in this context");
             return CSU_ERR_STATE;
         }
-        size_t per = (size_t)nv * nv;
+        const size_t per = (size_t)nv * nv, ne = block_entries(x->model), slots = x->max_ni;
+        const size_t total = (size_t)(nc + 31) / 32 * 32 * slots * ne;
         if (x->st.blocks) {
-            CK(d2h(a, x->st.blocks, (size_t)4 * per * nc));
+            CK(d2h(a, x->st.blocks, total));
         } else {
-            std::vector<float> f((size_t)4 * per * nc);
+            std::vector<float> f(total);
             CK(cudaMemcpy(f.data(), x->st.blocks32, sizeof(float) * f.size(), cudaMemcpyDeviceToHost));
             a.assign(f.begin(), f.end());
         }
+        // entries that are always zero, and slots no cell has, are not stored
+        memset(out, 0, sizeof(double) * (size_t)nc * 4 * per);
         for (int c = 0; c < nc; c++) {
             double* o = out + (size_t)n2o[c] * 4 * per;
-            for (int j = 0; j < 4; j++)
-                for (size_t e = 0; e < per; e++) o[j * per + e] = a[((size_t)j * per + e) * nc + c];
+            for (size_t j = 0; j < slots; j++) {
+                const double* e = a.data() + ((size_t)(c >> 5) * slots + j) * ne * 32 + (c & 31);
+                for (size_t q = 0; q < per; q++) {
+                    const int r = (int)(q / nv), k = (int)(q % nv);
+                    if (!block_nz(r, k)) continue;
+                    o[j * per + q] = *e;
+                    e += 32;
+                }
+            }
         }
         return CSU_OK;
     }

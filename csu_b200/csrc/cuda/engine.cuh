@@ -22,6 +22,33 @@ struct Model {
     static constexpr int NP = NV + 1;                                // primitives r u v p T (nt | k w)
 };
 
+// Entries of a DPLUR block that are not zero whatever the state: the mass flux depends on rho, rho u and rho v alone,
+// a transported scalar's on those and itself. (The momentum and energy fluxes hold the pressure, whose rounding the
+// finite difference keeps in every column.) 15 of 16, 22 of 25, 29 of 36; only these are stored and multiplied.
+__host__ __device__ constexpr bool block_nz(int r, int c)
+{
+    return r == 0 ? c < 3 : r < 4 || c < 3 || c == r;
+}
+
+// index of entry (r, c) among them, row by row; the number of them for (NV, 0)
+template <int MODEL>
+__host__ __device__ constexpr int block_entry(int r, int c)
+{
+    int n = 0;
+    for (int q = 0; q < r * Model<MODEL>::NV + c; q++) n += block_nz(q / Model<MODEL>::NV, q % Model<MODEL>::NV);
+    return n;
+}
+
+template <int MODEL>
+constexpr int BLOCK_NE = block_entry<MODEL>(Model<MODEL>::NV, 0);
+
+// Place of entry 0 of cell c's block across face slot j of `slots`: 32-cell tiles, in each [slot][entry][cell of 32].
+template <int MODEL>
+__host__ __device__ __forceinline__ size_t block_at(int c, int j, int slots)
+{
+    return ((size_t)(c >> 5) * slots + j) * (BLOCK_NE<MODEL> * 32) + (c & 31);
+}
+
 // Scalar settings, passed by value to every kernel.
 struct Prm {
     Gas gas;
@@ -136,8 +163,9 @@ struct State {
     double4* R4;  double* Rx;                 // residual
     double* dtl;                              // local steps (RK) or Omega / Lc (implicit)
     double* dpart;                            // implicit diagonal before Omega/dt
+    double* diag;                             // DPLUR: implicit diagonal with Omega/dt (first sweep)
     double4* X4[2]; double* Xx[2];            // DPLUR increments (ping-pong)
-    double* blocks;                           // DPLUR blocks [(slot*NV + row)*NV + col][cell]
+    double* blocks;                           // DPLUR blocks (block_at)
     float* blocks32;                          // the same in FP32 (mixed-precision DPLUR)
     double* part;                             // per-block partial sums of R^2 [block][NV]
     double* bcoef;                            // per reference boundary face: cp dSx, cp dSy, fx/q, fy/q

@@ -1122,7 +1122,7 @@ __global__ void __launch_bounds__(BLOCK) k_face_mit(const Prm* __restrict__ P, c
 // ------------------------------------------------------------------------------------------------
 template <int MODEL>
 __global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_blocks(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                                  const __grid_constant__ State s, int gb)
+                                                  const __grid_constant__ State s, int gb, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
     const int j = blockIdx.x / gb, cb = blockIdx.x - j * gb;
@@ -1197,13 +1197,54 @@ __global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_blocks(const Prm*
     }
 #pragma unroll
     for (int nn = 0; nn < NV; nn++) A[nn * NV + nn] -= 0.5 * ra;
-    const size_t base = (size_t)j * NV * NV * nc + c;
-    if (p.blk32) {
+    const size_t base = block_at<MODEL>(c, j, slots);
 #pragma unroll
-        for (int q = 0; q < NV * NV; q++) s.blocks32[base + (size_t)q * nc] = (float)A[q];
+    for (int q = 0; q < NV * NV; q++) {
+        if (!block_nz(q / NV, q % NV)) continue;
+        const size_t o = base + 32 * block_entry<MODEL>(q / NV, q % NV);
+        if (p.blk32) s.blocks32[o] = (float)A[q];
+        else s.blocks[o] = A[q];
+    }
+}
+
+// y += A x, terms in the reference's order (implicitMultA), the entries that are always zero left out
+template <int MODEL, typename T>
+__device__ __forceinline__ void block_times(const T* A, const double* x, double* y)
+{
+    constexpr int NV = Model<MODEL>::NV;
+#pragma unroll
+    for (int r = 0; r < NV; r++)
+#pragma unroll
+        for (int c = 0; c < NV; c++)
+            if (block_nz(r, c)) y[r] += (double)A[block_entry<MODEL>(r, c)] * x[c];
+}
+
+// the relaxed update of one cell from y = D x + sum_j A_j x_j (SST: the sum alone); D4: the SA variable's diagonal
+template <int MODEL>
+__device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, double D, double D4, const double* R,
+                                              const double* y, const double* xo, double* xn)
+{
+    constexpr int NV = Model<MODEL>::NV;
+    const double w = 2. / 3.;
+    if constexpr (MODEL == 2) {
+        // SST (extension): D on the mean flow; on k and omega, D minus the non-positive (destruction) part of the
+        // source Jacobians' diagonal, with their coupling to rho (the LU-SGS diagonal block, implicit.c:323-345,
+        // without its production part and k-omega cross terms, which made the iteration diverge at CFL 2 on
+        // wall-resolved meshes): x* = Dblock^-1 (-R - sum_j A_j x_j), then x += w (x* - x)
+        double z[NV], xs[NV];
+#pragma unroll
+        for (int k = 0; k < NV; k++) z[k] = -R[k] - y[k];
+#pragma unroll
+        for (int k = 0; k < 4; k++) xs[k] = z[k] / D;
+        const double a = D - fmin(s.dQ[(size_t)nc + c], 0.0);
+        const double dq = D - fmin(s.dQ[(size_t)5 * nc + c], 0.0);
+        xs[4] = (z[4] + s.dQ[c] * xs[0]) / a;
+        xs[5] = (z[5] + s.dQ[(size_t)3 * nc + c] * xs[0]) / dq;
+#pragma unroll
+        for (int k = 0; k < NV; k++) xn[k] = xo[k] + w * (xs[k] - xo[k]);
     } else {
 #pragma unroll
-        for (int q = 0; q < NV * NV; q++) s.blocks[base + (size_t)q * nc] = A[q];
+        for (int k = 0; k < NV; k++) xn[k] = w * (-R[k] - y[k]) / (k == 4 ? D4 : D) + xo[k];
     }
 }
 
@@ -1216,9 +1257,16 @@ __global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_blocks(const Prm*
 // the cell's residual R from the face fluxes (as k_impl does), stores it for the later sweeps and writes
 // the block's partial norms.
 // ------------------------------------------------------------------------------------------------
+//
+// Bound by HBM (or L2, when the blocks stay there) and the latency of the gathers. The blocks are stored without their
+// zeros in 32-cell tiles, each warp's a contiguous run (block_at): steady middle sweep of 160,000 triangles FP64
+// 16.5 -> 13.4 us, of 500,000 58 -> 47 us (244 MB, 5.2 TB/s, 79 % of the measured copy bandwidth), of the SA plate
+// (209,825 quads, FP32) 38.7 -> 23.8 us, SST airfoil pack 22 % faster per pass. SA's register budget is 96 (640
+// threads per SM): at the compiler's own 64 the plate's sweep takes 28.6 us, at 80 23.0 but the SA pack 5 % more;
+// Euler and SST are fastest at the compiler's choice (Euler held to 48: 16.7 us, SST held to 96 or 128: 2-5 % slower).
 template <int MODEL, bool LAST, bool FIRST, int SB, bool F32>
-__global__ void __launch_bounds__(SB) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                              const __grid_constant__ State s, int sweep, int cur)
+__global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+                                              const __grid_constant__ State s, int sweep, int cur, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
     static_assert(BLOCK % SB == 0, "sweep blocks tile the cell blocks");
@@ -1260,9 +1308,16 @@ __global__ void __launch_bounds__(SB) k_sweep(const Prm* __restrict__ P, const _
 #pragma unroll
             for (int k = 0; k < NV; k++) xn[k] = xo[k];
         } else {
-            double cfl = cfl_at(p, sc->iter);
-            double dt = p.implicit_local_dt ? s.dtl[c] * cfl : bitsd(sc->dtmin_bits) * cfl;
-            double D = s.dpart[c] + m.omega[c] / dt;
+            // the first sweep leaves the diagonal (implicitCalcD) for the others
+            double D;
+            if constexpr (FIRST) {
+                double cfl = cfl_at(p, sc->iter);
+                double dt = p.implicit_local_dt ? s.dtl[c] * cfl : bitsd(sc->dtmin_bits) * cfl;
+                D = s.dpart[c] + m.omega[c] / dt;
+                s.diag[c] = D;
+            } else {
+                D = s.diag[c];
+            }
             // y = D x + sum_j A_j x_j; SST keeps the off-diagonal sum alone (its diagonal is a block)
             double y[NV];
 #pragma unroll
@@ -1282,10 +1337,10 @@ __global__ void __launch_bounds__(SB) k_sweep(const Prm* __restrict__ P, const _
             int nbj[4];
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                int q = m.fnb[(size_t)j * nc + c];
+                int q = m.fnb[j * nc + c];
                 nbj[j] = q >= 0 ? q : c;
             }
-            nbj[3] = ni > 3 ? m.fnb[(size_t)3 * nc + c] : c;
+            nbj[3] = ni > 3 ? m.fnb[3 * nc + c] : c;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 if (j == 3 && ni <= 3) break;
@@ -1295,60 +1350,15 @@ __global__ void __launch_bounds__(SB) k_sweep(const Prm* __restrict__ P, const _
                 xb[0] = t.x; xb[1] = t.y; xb[2] = t.z; xb[3] = t.w;
 #pragma unroll
                 for (int k = 4; k < NV; k++) xb[k] = xox[(size_t)(k - 4) * nc + nb];
-                const size_t base = (size_t)j * NV * NV * nc + c;
+                const size_t base = block_at<MODEL>(c, j, slots);
                 const bool use = j < ni;
-                if constexpr (F32) {
-                    // FP32 blocks kept as floats until they are used: fewer registers, more cells in flight
-                    float Af[NV * NV];
+                double A[BLOCK_NE<MODEL>];
 #pragma unroll
-                    for (int q = 0; q < NV * NV; q++) Af[q] = s.blocks32[base + (size_t)q * nc];
-                    if (use) {
-#pragma unroll
-                        for (int kk = 0; kk < NV; kk++)
-#pragma unroll
-                            for (int nn = 0; nn < NV; nn++) y[kk] += (double)Af[kk * NV + nn] * xb[nn];
-                    }
-                } else {
-                    // FP64 blocks (the FP32 branch stays for contexts launched without F32: as compiled with
-                    // it, the FP64 sweep keeps more of its loads in flight than an FP64-only build does)
-                    double A[NV * NV];
-                    if (p.blk32) {
-#pragma unroll
-                        for (int q = 0; q < NV * NV; q++) A[q] = (double)s.blocks32[base + (size_t)q * nc];
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < NV * NV; q++) A[q] = s.blocks[base + (size_t)q * nc];
-                    }
-                    if (use) {
-#pragma unroll
-                        for (int kk = 0; kk < NV; kk++)
-#pragma unroll
-                            for (int nn = 0; nn < NV; nn++) y[kk] += A[kk * NV + nn] * xb[nn];
-                    }
-                }
+                for (int q = 0; q < BLOCK_NE<MODEL>; q++)
+                    A[q] = F32 ? (double)s.blocks32[base + 32 * q] : s.blocks[base + 32 * q];
+                if (use) block_times<MODEL>(A, xb, y);
             }
-            const double w = 2. / 3.;
-            if constexpr (MODEL == 2) {
-                // SST (extension): D on the mean flow; on k and omega, D minus the non-positive (destruction)
-                // part of the source Jacobians' diagonal, with their coupling to rho (the LU-SGS diagonal
-                // block, implicit.c:323-345, without its production part and k-omega cross terms, which made
-                // the iteration diverge at CFL 2 on wall-resolved meshes): x* = Dblock^-1 (-R - sum_j A_j x_j),
-                // then x += w (x* - x)
-                double z[NV], xs[NV];
-#pragma unroll
-                for (int k = 0; k < NV; k++) z[k] = -R[k] - y[k];
-#pragma unroll
-                for (int k = 0; k < 4; k++) xs[k] = z[k] / D;
-                const double a = D - fmin(s.dQ[(size_t)nc + c], 0.0);
-                const double dq = D - fmin(s.dQ[(size_t)5 * nc + c], 0.0);
-                xs[4] = (z[4] + s.dQ[c] * xs[0]) / a;
-                xs[5] = (z[5] + s.dQ[(size_t)3 * nc + c] * xs[0]) / dq;
-#pragma unroll
-                for (int k = 0; k < NV; k++) xn[k] = xo[k] + w * (xs[k] - xo[k]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < NV; k++) xn[k] = w * (-R[k] - y[k]) / (k == 4 ? D4 : D) + xo[k];
-            }
+            jacobi_update<MODEL>(s, nc, c, D, D4, R, y, xo, xn);
             dmax = fabs(xn[0] - xo[0]);
         }
         xn4[c] = make_double4(xn[0], xn[1], xn[2], xn[3]);
