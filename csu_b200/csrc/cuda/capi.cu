@@ -1128,12 +1128,12 @@ static void launch_iteration(csu_ctx* x)
                 int col = pass == 0 ? q : K - 1 - q;
                 int start = x->L.color_start[col], count = x->L.color_start[col + 1] - start;
                 if (count == 0) continue;
-                int g = (count + BLOCK - 1) / BLOCK;
+                int g = (int)(((long long)count * 4 + LUSGS_THREADS - 1) / LUSGS_THREADS);
                 if (pass == 0)
-                    k_lusgs<MODEL, true><<<g, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st, x->mesh.color,
+                    k_lusgs<MODEL, true><<<g, LUSGS_THREADS, 0, x->stream>>>(x->d_prm, x->mesh, x->st, x->mesh.color,
                                                                      x->mesh.color_cells, col, start, count);
                 else
-                    k_lusgs<MODEL, false><<<g, BLOCK, 0, x->stream>>>(x->d_prm, x->mesh, x->st, x->mesh.color,
+                    k_lusgs<MODEL, false><<<g, LUSGS_THREADS, 0, x->stream>>>(x->d_prm, x->mesh, x->st, x->mesh.color,
                                                                       x->mesh.color_cells, col, start, count);
                 x->launches++;
                 tmark(x, KSWEEP);
