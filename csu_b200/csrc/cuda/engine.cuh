@@ -181,6 +181,21 @@ struct State {
 
 // ---------------------------------------------------------------- small helpers
 
+// Programmatic dependent launch: a kernel launched with the attribute starts while the one before it in the stream
+// still runs and must not touch anything an iteration writes until pdl_wait, past which every earlier kernel is done
+// and visible. Every kernel of the chain waits before it lets the next one start, so what runs before a wait runs
+// beside one kernel at most. Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+__device__ __forceinline__ void prefetch_l1(const void* p)
+{
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 __device__ __forceinline__ unsigned long long dbits(double x)
 {
     return (unsigned long long)__double_as_longlong(x);

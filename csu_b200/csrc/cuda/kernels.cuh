@@ -194,6 +194,7 @@ __device__ __noinline__ double lsq_slot_x87(const Prm& p, const Mesh& m, const S
 __global__ void k_minmax_init(State s)
 {
     Scalars* sc = s.sc + blockIdx.x;
+    pdl_wait();
     if (threadIdx.x < 6) {
         sc->qmin_bits[threadIdx.x] = ~0ULL;
         sc->qmax_bits[threadIdx.x] = 0ULL;
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(BLOCK) k_minmax(const Prm* __restrict__ P, con
     const int sid = block_solve(s);
     const Prm& p = P[sid];
     Scalars* const sc = s.sc + sid;
+    pdl_wait();
     if (halted_behind(p, sc)) return;
     const int c = blockIdx.x * BLOCK + threadIdx.x;
     const bool ok = cell_in(p, c);
@@ -297,30 +299,32 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), grad_bloc
     const int nc = m.nc; // 4 nc < 2^31
     if (LSQ == 2 && threadIdx.x == 0) nlist = 0;
     if (LSQ == 2) __syncthreads();
-    if (cell_in(p, c) && !halted_behind(p, sc)) {
-        const double* const W = kk < 4 ? reinterpret_cast<const double*>(s.W4) + kk
-                                       : vi == 4 ? s.WT : s.Wx + (size_t)(vi - 5) * nc;
-        const int ws = kk < 4 ? 4 : 1;
-        const double u0 = W[(size_t)c * ws];
-        const int np = m.npts[c];
-        int nj[4];
-        double2 d[4];
+    // the mesh rows before the wait for the previous kernel (padding rows are in bounds and hold zeros)
+    const double* const W = kk < 4 ? reinterpret_cast<const double*>(s.W4) + kk
+                                   : vi == 4 ? s.WT : s.Wx + (size_t)(vi - 5) * nc;
+    const int ws = kk < 4 ? 4 : 1;
+    const int cr = min(c, nc - 1), np = m.npts[cr];
+    int nj[4];
+    double2 d[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (j < 3 || np > 3) {
-                nj[j] = m.nei[j * nc + c];
-                d[j] = (LSQ == 0 ? m.lw : m.ld)[j * nc + c];
-            }
+    for (int j = 0; j < 4; j++) {
+        nj[j] = cr;
+        if (j < 3 || np > 3) {
+            nj[j] = m.nei[j * nc + cr];
+            d[j] = (LSQ == 0 ? m.lw : m.ld)[j * nc + cr];
         }
-        double un[4] = {u0, u0, u0, u0};
-        unsigned ghosts = 0;
+    }
+    pdl_wait();
+    const bool stop = halted_behind(p, sc);
+    const double u0 = W[(size_t)cr * ws];
+    double un[4];
+    unsigned ghosts = 0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (j < 3 || np > 3) {
-                if (nj[j] < nc) un[j] = W[(size_t)nj[j] * ws];
-                else ghosts |= 1u << j;
-            }
-        }
+    for (int j = 0; j < 4; j++) {
+        un[j] = W[(size_t)(nj[j] < nc ? nj[j] : cr) * ws];
+        if (nj[j] >= nc) ghosts |= 1u << j;
+    }
+    if (cell_in(p, c) && !stop) {
         if (ghosts) {
             double P0[NP], Pn[NP];
             loadP<MODEL>(s, nc, c, P0);
@@ -674,15 +678,23 @@ __global__ void __launch_bounds__(FB) k_flux(const Prm* __restrict__ P, const __
         int2 e = m.fe[f];
         const int sid = cell_solve(s, e.x);
         const Prm& p = P[sid];
+        const bool o2 = p.order == 2, grad = o2 || p.visc;
+        prefetch_l1(m.fn + f);
+        prefetch_l1(m.fds + f);
+        if (o2) {
+            prefetch_l1(m.r0 + f);
+            prefetch_l1(m.r1 + f);
+        }
+        pdl_wait();
         if (halted_behind(p, s.sc + sid)) return;
         const double4 z4 = make_double4(0.0, 0.0, 0.0, 0.0);
-        const bool grad = p.order == 2 || p.visc;
         interior_face<MODEL>(p, m, s, f, e, s.W4[e.x], s.WT[e.x], grad ? s.G4x[e.x] : z4, grad ? s.G4y[e.x] : z4,
-                             p.order == 2 ? s.PH4[e.x] : z4, s.W4[e.y], s.WT[e.y], grad ? s.G4x[e.y] : z4,
-                             grad ? s.G4y[e.y] : z4, p.order == 2 ? s.PH4[e.y] : z4);
+                             o2 ? s.PH4[e.x] : z4, s.W4[e.y], s.WT[e.y], grad ? s.G4x[e.y] : z4,
+                             grad ? s.G4y[e.y] : z4, o2 ? s.PH4[e.y] : z4);
     } else {
         int b = (blockIdx.x - nbi) * FB + threadIdx.x;
         if (b >= m.nb) return;
+        pdl_wait();
         boundary_face<MODEL>(P, m, s, b, wall_rank, coef);
     }
 }
@@ -700,6 +712,7 @@ __global__ void __launch_bounds__(FB) k_flux_st(const Prm* __restrict__ P, const
                                                 const __grid_constant__ State s, int nbi, const int* wall_rank,
                                                 int coef)
 {
+    pdl_wait();
     if ((int)blockIdx.x >= nbi) {
         const int b = (blockIdx.x - nbi) * FB + threadIdx.x;
         if (b < m.nb) boundary_face<MODEL>(P, m, s, b, wall_rank, coef);
@@ -919,9 +932,18 @@ __global__ void __launch_bounds__(BLOCK) k_rk(const Prm* __restrict__ P, const _
     const int sid = block_solve(s);
     const Prm& p = P[sid];
     Scalars* const sc = s.sc + sid;
-    if (halted(sc)) return;
     int c = blockIdx.x * BLOCK + threadIdx.x;
     bool valid = cell_in(p, c);
+    if (valid) {
+        // mesh rows before the wait for the previous kernel
+        prefetch_l1(m.nslot + c);
+        prefetch_l1(m.omega + c);
+        if (p.visc) prefetch_l1(m.nint + c);
+#pragma unroll
+        for (int j = 0; j < 4; j++) prefetch_l1(m.fslot + j * m.nc + c);
+    }
+    pdl_wait();
+    if (halted(sc)) return;
     double R[NV];
     double lmin = bitsd(0x7ff0000000000000ULL);
     if (valid) {
@@ -978,9 +1000,10 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
     const int sid = block_solve(s);
     const Prm& p = P[sid];
     Scalars* const sc = s.sc + sid;
-    if (halted(sc)) return;
     int c = blockIdx.x * BLOCK + threadIdx.x;
     bool valid = cell_in(p, c);
+    pdl_wait();
+    if (halted(sc)) return;
     double R[NV];
     double lmin = bitsd(0x7ff0000000000000ULL);
     if (valid) {
@@ -1274,12 +1297,26 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
     const int sid = s.bsolve ? s.bsolve[blockIdx.x / (BLOCK / SB)] : 0;
     const Prm& p = P[sid];
     Scalars* const sc = s.sc + sid;
-    if (halted(sc)) return;
     int c = blockIdx.x * SB + threadIdx.x;
     const int nc = m.nc;
+    const bool valid = cell_in(p, c);
+    // Slots 0-2 are gathered unconditionally (a slot without a face reads the cell itself and a zero block, both in
+    // bounds, and is not summed), so their index and neighbour loads issue together instead of one dependent chain
+    // per face; slot 3 only exists in quadrilaterals. The indices are read before the wait for the previous sweep.
+    int ni = 0, nbj[4] = {c, c, c, c};
+    if (valid) {
+        ni = m.nint[c];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            int q = m.fnb[j * nc + c];
+            nbj[j] = q >= 0 ? q : c;
+        }
+        if (ni > 3) nbj[3] = m.fnb[3 * nc + c];
+    }
+    pdl_wait();
+    if (halted(sc)) return;
     bool conv = !FIRST && sweep > 0 && bitsd(sc->sweep_max[sweep - 1]) < 1e-14;
     double dmax = 0.0;
-    const bool valid = cell_in(p, c);
     double R[NV];
     if (valid) {
         const double4* xo4 = s.X4[cur];
@@ -1330,17 +1367,6 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
                     y[4] = D4 * xo[4];
                 }
             }
-            // Slots 0-2 are gathered unconditionally (a slot without a face reads the cell itself and a zero
-            // block, both in bounds, and is not summed), so their index and neighbour loads issue together
-            // instead of one dependent chain per face; slot 3 only exists in quadrilaterals.
-            const int ni = m.nint[c];
-            int nbj[4];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                int q = m.fnb[j * nc + c];
-                nbj[j] = q >= 0 ? q : c;
-            }
-            nbj[3] = ni > 3 ? m.fnb[3 * nc + c] : c;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 if (j == 3 && ni <= 3) break;
@@ -1490,11 +1516,12 @@ __global__ void __launch_bounds__(LUSGS_THREADS) k_lusgs(const Prm* __restrict__
     const int sid = cell_solve(s, c);
     const Prm& p = P[sid];
     Scalars* const sc = s.sc + sid;
-    const bool store = t < count && !halted(sc);
     const int sf = m.fslot[j * nc + c];
     const int nb = max(m.fnb[j * nc + c], 0);
     const bool use = j < m.nint[c];
     const int cn = color[nb];
+    pdl_wait();
+    const bool store = t < count && !halted(sc);
     const double4* src4 = FWD ? s.X4[0] : s.X4[1];
     const double* srcx = FWD ? s.Xx[0] : s.Xx[1];
     const double cfl = cfl_at(p, sc->iter);
@@ -1611,6 +1638,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(const Prm* __restrict__ P, con
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
     const Prm& p = P[block_solve(s)];
+    pdl_wait();
     if (halted(s.sc + block_solve(s))) return;
     int c = blockIdx.x * BLOCK + threadIdx.x;
     if (!cell_in(p, c)) return;
@@ -1648,6 +1676,7 @@ __global__ void __launch_bounds__(BLOCK) k_finalize(const Prm* __restrict__ P, c
     // Everything the block reads is requested before the halted test, so the loads overlap: a chain of
     // dependent round trips to the L2 would be most of a one-block kernel's time. Thread 0 keeps a copy of
     // the solve's scalars and writes back only what changes.
+    pdl_wait();
     const bool stop = mode != 2 && mode != 3 && halted(sc);
     double v[NV + 4];
 #pragma unroll
