@@ -257,6 +257,7 @@ static void plan(csu_ctx* x, Arena& a)
     m.dslat = carve<double>(a, nc);
     m.fe = carve<int2>(a, nf);
     m.fn = carve<double2>(a, nf);
+    m.fun = carve<double2>(a, nf);
     m.fds = carve<double>(a, nf);
     m.r0 = carve<double2>(a, nf);
     m.r1 = carve<double2>(a, nf);
@@ -305,6 +306,10 @@ static void plan(csu_ctx* x, Arena& a)
     }
     bool dplur = x->cfg.time_scheme == CSU_TS_DPLUR;
     s.diag = dplur ? carve<double>(a, nc) : nullptr;
+    s.PR4 = dplur ? carve<double4>(a, nc) : nullptr;
+    s.PRx = dplur && x->cfg.sst ? carve<double>(a, nc) : nullptr;
+    s.FR = dplur ? carve<double2>(a, nf) : nullptr;
+    s.FB = dplur && visc ? carve<double>(a, nf) : nullptr;
     const size_t nblocks = (size_t)(nc + 31) / 32 * 128 * block_entries(x->model);
     s.blocks = dplur && !x->cfg.implicit_fp32 ? carve<double>(a, nblocks) : nullptr;
     s.blocks32 = dplur && x->cfg.implicit_fp32 ? carve<float>(a, nblocks) : nullptr;
@@ -338,11 +343,12 @@ static int upload_mesh(csu_ctx* x)
         return cudaMemcpy(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice);
     };
     std::vector<int2> fe(nf);
-    std::vector<double2> fn(nf), r0(nf), r1(nf), bn(nb), fd(nf), bd(nb), bun(nb);
+    std::vector<double2> fn(nf), fun(nf), r0(nf), r1(nf), bn(nb), fd(nf), bd(nb), bun(nb);
     for (int f = 0; f < nf; f++) {
         fe[f] = make_int2(L.fe0[f], L.fe1[f]);
         fd[f] = make_double2(L.fdx[f], L.fdy[f]);
         fn[f] = make_double2(L.fdsx[f], L.fdsy[f]);
+        fun[f] = make_double2(L.fdsx[f] / L.fds[f], L.fdsy[f] / L.fds[f]);
         r0[f] = make_double2(L.r0x[f], L.r0y[f]);
         r1[f] = make_double2(L.r1x[f], L.r1y[f]);
     }
@@ -401,6 +407,7 @@ static int upload_mesh(csu_ctx* x)
     CK(up(m.dslat, L.dslat, sizeof(double) * nc));
     CK(up(m.fe, fe.data(), sizeof(int2) * nf));
     CK(up(m.fn, fn.data(), sizeof(double2) * nf));
+    CK(up(m.fun, fun.data(), sizeof(double2) * nf));
     CK(up(m.fds, L.fds, sizeof(double) * nf));
     CK(up(m.r0, r0.data(), sizeof(double2) * nf));
     CK(up(m.r1, r1.data(), sizeof(double2) * nf));
@@ -428,6 +435,8 @@ static void fill_params_from(const csu_config& c, const csu_layout& L, Prm& p)
     p.gas.R = c.gas_r;
     p.gas.Cp = c.gamma * c.gas_r / (c.gamma - 1); // gaspropInit (gasprop.c:14-37)
     p.gas.Cv = p.gas.Cp - c.gas_r;
+    p.gas.gam = (p.gas.Cv + p.gas.R) / p.gas.Cv;
+    p.gas.gamR = p.gas.gam * p.gas.R;
     p.gas.tp = c.tp;
     p.nc = L.nc;
     p.nf = L.nf;
@@ -1042,9 +1051,9 @@ static void launch_prologue(csu_ctx* x)
 // the caller before the kernels they run beside, which are launched first so that their blocks are dispatched
 // first and k_blocks fills the SMs their last wave leaves idle); the first sweep joins. Timed runs keep them
 // on the engine stream, so each kernel kind's events bracket it alone.
-// The implicit diagonal and step (k_impl without R) go on the same side stream. SA first computes the face
-// eddy viscosity the blocks and the diagonal use (k_face_mit); with saImplicitSource its diagonal also needs
-// the gradients, so k_impl waits for ev_grad (recorded after them).
+// The implicit diagonal and step (k_impl without R) go on the same side stream, after what both use per cell and face
+// (k_side); with saImplicitSource SA's diagonal also needs the gradients, so k_impl waits for ev_grad (recorded after
+// them).
 template <int MODEL>
 static void launch_blocks(csu_ctx* x)
 {
@@ -1053,10 +1062,8 @@ static void launch_blocks(csu_ctx* x)
         cudaStreamWaitEvent(x->side, x->ev_fork, 0);
         s = x->side;
     }
-    if (MODEL == 1 && x->prm.mit_early) {
-        k_face_mit<<<(x->L.nf + BLOCK - 1) / BLOCK, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st);
-        x->launches++;
-    }
+    k_side<MODEL><<<x->gb_c + (x->L.nf + BLOCK - 1) / BLOCK, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st, x->gb_c);
+    x->launches++;
     k_blocks<MODEL><<<x->max_ni * x->gb_c, BLOCK, 0, s>>>(x->d_prm, x->mesh, x->st, x->gb_c, x->max_ni);
     x->launches++;
     if (x->timing) tmark(x, KBLK);
@@ -1164,7 +1171,7 @@ static void launch_iteration(csu_ctx* x)
         launch_finalize<MODEL>(x, 1);
     } else {
         // the SST blocks and diagonal need the face eddy viscosity of k_flux (and the gradients, for the
-        // source Jacobians); the SA ones only k_face_mit's, the Euler/laminar ones the iteration's start state
+        // source Jacobians); the SA ones only k_side's, the Euler/laminar ones the iteration's start state
         constexpr bool early = MODEL <= 1;
         const bool grad = c.order == 2 || x->prm.visc;
         // Inside a captured graph an iteration's k_finalize (norms, history row, halt flags, counters) runs on
@@ -2224,7 +2231,7 @@ static std::vector<SegArr> seg_arrays(csu_ctx* x)
         {P(m.lk), 16, SEG_CELL3}, {P(m.em), 16, SEG_CELL4}, {P(m.fslot), 4, SEG_CELL4}, {P(m.fnb), 4, SEG_CELL4},
         {P(m.omega), 8, SEG_CELL}, {P(m.sxh), 8, SEG_CELL}, {P(m.syh), 8, SEG_CELL},
         {P(m.dslat), 8, SEG_CELL}, {P(m.color), 4, SEG_CELL},
-        {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE}, {P(m.r0), 16, SEG_FACE},
+        {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fun), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE}, {P(m.r0), 16, SEG_FACE},
         {P(m.r1), 16, SEG_FACE}, {P(m.fd), 16, SEG_FACE}, {P(m.fL), 8, SEG_FACE},
         {P(m.bown), 4, SEG_BFACE}, {P(m.bflag), 4, SEG_BFACE}, {P(m.bold), 4, SEG_BFACE},
         {P(m.bn), 16, SEG_BFACE}, {P(m.bds), 8, SEG_BFACE}, {P(m.bd), 16, SEG_BFACE}, {P(m.bL), 8, SEG_BFACE},
@@ -2257,6 +2264,12 @@ static std::vector<const void*> seg_host(const csu_layout& L, std::vector<std::v
         for (int i = 0; i < n; i++) d[i] = make_double2(a[i], b[i]);
         return (const void*)d;
     };
+    auto unit = [&]() {
+        keep.emplace_back((size_t)nf * sizeof(double2) + 1);
+        double2* d = (double2*)keep.back().data();
+        for (int i = 0; i < nf; i++) d[i] = make_double2(L.fdsx[i] / L.fds[i], L.fdsy[i] / L.fds[i]);
+        return (const void*)d;
+    };
     keep.emplace_back((size_t)nf * sizeof(int2) + 1);
     int2* fe = (int2*)keep.back().data();
     for (int f = 0; f < nf; f++) fe[f] = make_int2(L.fe0[f], L.fe1[f]);
@@ -2266,7 +2279,7 @@ static std::vector<const void*> seg_host(const csu_layout& L, std::vector<std::v
     std::vector<const void*> v = {
         L.npts, L.nint, L.nslot, L.nei, L.lw, L.ld, L.lm, L.les, L.lrv, L.lq, L.lk, L.em, L.fslot, L.fnb,
         L.omega, L.sxh, L.syh, L.dslat, L.color,
-        fe, pairs(L.fdsx, L.fdsy, nf), L.fds, pairs(L.r0x, L.r0y, nf), pairs(L.r1x, L.r1y, nf),
+        fe, pairs(L.fdsx, L.fdsy, nf), unit(), L.fds, pairs(L.r0x, L.r0y, nf), pairs(L.r1x, L.r1y, nf),
         pairs(L.fdx, L.fdy, nf), L.fdist,
         L.bown, L.bflag, L.bold, pairs(L.bdsx, L.bdsy, nb), L.bds, pairs(L.bdx, L.bdy, nb), L.bL,
         pairs(L.bunx, L.buny, nb), L.bds2, rank};

@@ -75,7 +75,7 @@ struct Prm {
     int blk32;          // DPLUR blocks in FP32
     int sa_isrc;        // SA + DPLUR: the source's implicit part in the nt diagonal (dQ holds it per cell)
     int defer_fin;      // DPLUR: an iteration's k_finalize may run beside the next one's gradients and fluxes
-    int mit_early;      // SA + DPLUR: k_face_mit writes the face eddy viscosity (from the primitives alone) for
+    int mit_early;      // SA + DPLUR: k_side writes the face eddy viscosity (from the primitives alone) for
                         // the blocks and the diagonal, which then need not wait for k_flux; k_flux skips it
     int implicit_local_dt;
     int cfl_ramp_iters; // CFL ramp (0: constant CFL)
@@ -132,6 +132,7 @@ struct Mesh {
     const double* dslat;
     const int2* fe;
     const double2* fn;
+    const double2* fun;             // fn / fds
     const double* fds;
     const double2* r0;
     const double2* r1;
@@ -163,6 +164,9 @@ struct State {
     double4* R4;  double* Rx;                 // residual
     double* dtl;                              // local steps (RK) or Omega / Lc (implicit)
     double* dpart;                            // implicit diagonal before Omega/dt
+    double4* PR4; double* PRx;                // DPLUR: pressures of the finite differences' states (k_side)
+    double2* FR; double* FB;                  // DPLUR: per interior face, convective radius times |dS| and viscous
+                                              // radius times |dS|^2; viscous radius times |dS| over |fd| (k_side)
     double* diag;                             // DPLUR: implicit diagonal with Omega/dt (first sweep)
     double4* X4[2]; double* Xx[2];            // DPLUR increments (ping-pong)
     double* blocks;                           // DPLUR blocks (block_at)

@@ -987,6 +987,32 @@ __device__ __forceinline__ void aux_flux(const double* U, double pr, double nx, 
     for (int k = 4; k < NV; k++) F[k] = U[k] * V;
 }
 
+// Convective spectral radius of interior face f times |dS|, and the viscous one (0 inviscid) times |dS|, from the face
+// means of the two cells (implicitCalcD, implicit.c:19-181).
+template <int MODEL>
+__device__ __forceinline__ void face_radii(const Prm& p, const Mesh& m, const State& s, int f, double* Lc, double* Lv)
+{
+    const int2 e = m.fe[f];
+    const double4 w0 = s.W4[e.x], w1 = s.W4[e.y];
+    const double T0 = s.WT[e.x], T1 = s.WT[e.y];
+    const double2 un = m.fun[f];
+    const double dS = m.fds[f];
+    double u = (w0.y + w1.y) * 0.5;
+    double v = (w0.z + w1.z) * 0.5;
+    double T = (T0 + T1) * 0.5;
+    double cc = T2c(p.gas, T);
+    *Lc = (fabs(un.x * u + un.y * v) + cc) * dS;
+    *Lv = 0.0;
+    if constexpr (MODEL >= 1) {
+        double r = (w0.x + w1.x) * 0.5;
+        double mi = sutherland(T);
+        *Lv = fmax(4 / (3 * r), T2gamma(p.gas, T) / r) * (mi / p.pr + s.MIT[f] / p.pr_t) * dS;
+    } else if (p.laminar) {
+        double r = (w0.x + w1.x) * 0.5;
+        *Lv = visc_radius(p.gas, p.pr, r, T) * dS;
+    }
+}
+
 // ------------------------------------------------------------------------------------------------
 // k_impl: R (WITH_R) and the implicit diagonal (implicitCalcD, implicit.c:19-181) of each cell. The
 // diagonal, the local steps and their minimum need only the iteration's start state, so DPLUR computes them
@@ -1051,27 +1077,30 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
         }
         const int ni = m.nint[c], ns = m.nslot[c];
         double Lc = 0, Lv = 0;
-        for (int j = 0; j < ni; j++) {
-            int sf = m.fslot[(size_t)j * nc + c];
-            int f = sf > 0 ? sf - 1 : -sf - 1;
-            int2 e = m.fe[f];
-            double4 w0 = s.W4[e.x], w1 = s.W4[e.y];
-            double T0 = s.WT[e.x], T1 = s.WT[e.y];
-            double2 dSv = m.fn[f];
-            double dS = m.fds[f];
-            double u = (w0.y + w1.y) * 0.5;
-            double v = (w0.z + w1.z) * 0.5;
-            double T = (T0 + T1) * 0.5;
-            double cc = T2c(p.gas, T);
-            double nx = dSv.x / dS, ny = dSv.y / dS;
-            Lc += (fabs(nx * u + ny * v) + cc) * dS;
-            if constexpr (MODEL >= 1) {
-                double r = (w0.x + w1.x) * 0.5;
-                double mi = sutherland(T);
-                Lv += fmax(4 / (3 * r), T2gamma(p.gas, T) / r) * (mi / p.pr + s.MIT[f] / p.pr_t) * dS * dS;
-            } else if (p.laminar) {
-                double r = (w0.x + w1.x) * 0.5;
-                Lv += visc_radius(p.gas, p.pr, r, T) * dS * dS;
+        if constexpr (WITH_R) {
+            for (int j = 0; j < ni; j++) {
+                int sf = m.fslot[(size_t)j * nc + c];
+                double Lcf, Lvf;
+                face_radii<MODEL>(p, m, s, sf > 0 ? sf - 1 : -sf - 1, &Lcf, &Lvf);
+                Lc += Lcf;
+                Lv += Lvf * m.fds[sf > 0 ? sf - 1 : -sf - 1];
+            }
+        } else {
+            // DPLUR: k_side's, one gather per face
+            double2 fr[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (j < ni) {
+                    const int sf = m.fslot[j * nc + c];
+                    fr[j] = s.FR[(sf > 0 ? sf : -sf) - 1];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (j < ni) {
+                    Lc += fr[j].x;
+                    Lv += fr[j].y;
+                }
             }
         }
         double D = 0.5 * p.w_imp * Lc;
@@ -1108,43 +1137,119 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
     if (WITH_R) partial_norms<MODEL>(s, valid, R);
 }
 
-// ------------------------------------------------------------------------------------------------
-// k_face_mit: the SA face eddy viscosity mu_t = fv1 rho nt of the face means of the two cells' primitives
-// (saBoundaryVisc's interior part, sa.c: the same expressions as sa_face_flux / sacc_face_flux, whose value
-// it equals bit for bit), for the DPLUR blocks and diagonal: it needs no gradient, so they can run beside
-// k_grad and k_flux instead of after them.
-// ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(BLOCK) k_face_mit(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                                    const __grid_constant__ State s)
+// Step of the blocks' finite difference in variable mm (implicit.c:692). SST: rho omega reaches 1e10 beside a wall, where
+// a step of 1e-6 is below its last bit; its column (a flux linear in rho omega) and rho k's take a step relative to the
+// value.
+constexpr double BLOCK_H = 1.0e-6;
+
+template <int MODEL>
+__device__ __forceinline__ double pert_step(int mm, const double* U)
 {
-    const int f = blockIdx.x * BLOCK + threadIdx.x;
-    if (f >= m.nf) return;
-    const int2 e = m.fe[f];
-    const int sid = cell_solve(s, e.x);
-    if (halted(s.sc + sid)) return;
-    const int nc = m.nc;
-    const double4 w0 = s.W4[e.x], w1 = s.W4[e.y];
-    const double r = (w1.x + w0.x) * 0.5;
-    const double T = (s.WT[e.y] + s.WT[e.x]) * 0.5;
-    const double n = (s.Wx[e.y] + s.Wx[e.x]) * 0.5;
-    const double mi_L = sutherland(T);
-    const double n_L = mi_L / r;
-    double fv1, tx, ty;
-    sa_face(n, n_L, r, 0.0, 0.0, &fv1, &tx, &ty);
-    s.MIT[f] = fv1 * r * n;
-    (void)nc;
+    return MODEL == 2 && mm >= 4 ? BLOCK_H * fmax(1.0, fabs(U[mm])) : BLOCK_H;
+}
+
+// a / BLOCK_H, correctly rounded, by the divisor's reciprocal as a double-double: q = RN(a zh + RN(a zl)) (Brisebarre,
+// Muller & Raina, "Accelerating correctly rounded floating-point division when the divisor is known in advance", IEEE
+// Trans. Computers 53, 2004) is within 2^-105 of the quotient, and no quotient of a double by this divisor whose
+// rounding that could change does change (tests/test_block_step.py checks every one). Zeros keep their sign; outside
+// the exponents where the products are exact enough, the division itself, out of line.
+static __host__ __device__ __noinline__ double over_h_any(double a)
+{
+    return a / BLOCK_H;
+}
+
+__host__ __device__ __forceinline__ double over_h(double a)
+{
+    const double zh = 0x1.e848p+19, zl = 0x1.8e0a318p-35;
+    const double m = fabs(a);
+    if (m == 0.0 || (m >= 0x1p-900 && m <= 0x1p+900)) return fma(a, zh, a * zl);
+    return over_h_any(a);
+}
+
+// ------------------------------------------------------------------------------------------------
+// k_side: what the DPLUR blocks and diagonal need once per cell or face, before them on the side stream. The first gc
+// blocks: the pressures of a cell's states with one conserved variable stepped (implicitUpdateA, implicit.c:692-788),
+// 14 divisions per cell instead of per block. The others: a face's spectral radii, which both cells' diagonals and both
+// its blocks use, and for SA the face eddy viscosity mu_t = fv1 rho nt of the face means of the two cells' primitives
+// (saBoundaryVisc's interior part, sa.c: the same expressions as sa_face_flux / sacc_face_flux, whose value it equals
+// bit for bit): it needs no gradient, so the blocks and the diagonal can run beside k_grad and k_flux.
+// ------------------------------------------------------------------------------------------------
+template <int MODEL>
+__global__ void __launch_bounds__(BLOCK) k_side(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+                                                const __grid_constant__ State s, int gc)
+{
+    constexpr int NV = Model<MODEL>::NV, NM = MODEL == 2 ? 5 : 4;
+    if ((int)blockIdx.x >= gc) {
+        const int f = (blockIdx.x - gc) * BLOCK + threadIdx.x;
+        if (f >= m.nf) return;
+        const int2 e = m.fe[f];
+        const int sid = cell_solve(s, e.x);
+        const Prm& p = P[sid];
+        if (halted(s.sc + sid)) return;
+        if constexpr (MODEL == 1) {
+            const double r = (s.W4[e.y].x + s.W4[e.x].x) * 0.5;
+            const double T = (s.WT[e.y] + s.WT[e.x]) * 0.5;
+            const double n = (s.Wx[e.y] + s.Wx[e.x]) * 0.5;
+            const double mi_L = sutherland(T);
+            const double n_L = mi_L / r;
+            double fv1, tx, ty;
+            sa_face(n, n_L, r, 0.0, 0.0, &fv1, &tx, &ty);
+            s.MIT[f] = fv1 * r * n;
+        }
+        double Lc, Lv;
+        face_radii<MODEL>(p, m, s, f, &Lc, &Lv);
+        s.FR[f] = make_double2(Lc, Lv * m.fds[f]);
+        if (s.FB) s.FB[f] = Lv / m.fL[f];
+        return;
+    }
+    const int sid = block_solve(s);
+    const Prm& p = P[sid];
+    const int c = blockIdx.x * BLOCK + threadIdx.x;
+    if (!cell_in(p, c) || halted(s.sc + sid)) return;
+    double U[NV], Uq[NV], pr[NM];
+    loadU<MODEL>(s, m.nc, c, U);
+    const double T0 = s.WT[c];
+    double rho = U[0];
+    double uu = U[1] / rho;
+    double vv = U[2] / rho;
+    double E = U[3] / rho;
+    double ee0 = E - 0.5 * (uu * uu + vv * vv);
+    // SST (an extension: the reference's SST DPLUR multiplies 4x4 blocks into six variables, implicit.c:
+    // 990-1000 with 938-972): the energy holds the turbulent kinetic energy, as in its SST delta flux
+    // (implicitCalcDeltaFlux_sst, implicit.c:1048-1118)
+    if constexpr (MODEL == 2) ee0 = ee0 - U[4] / rho;
+#pragma unroll
+    for (int mm = 0; mm < NM; mm++) {
+        const double hm = pert_step<MODEL>(mm, U);
+#pragma unroll
+        for (int nn = 0; nn < NV; nn++) Uq[nn] = mm == nn ? U[nn] + hm : U[nn];
+        double r2 = Uq[0];
+        double u2 = Uq[1] / r2;
+        double v2 = Uq[2] / r2;
+        double E2 = Uq[3] / r2;
+        double ee1 = E2 - 0.5 * (u2 * u2 + v2 * v2);
+        if constexpr (MODEL == 2) ee1 = ee1 - Uq[4] / r2;
+        double T = e2Taprox(p.gas, ee0, T0, ee1);
+        pr[mm] = p.gas.R * r2 * T;
+    }
+    s.PR4[c] = make_double4(pr[0], pr[1], pr[2], pr[3]);
+    if constexpr (MODEL == 2) s.PRx[c] = pr[4];
 }
 
 // ------------------------------------------------------------------------------------------------
 // k_blocks: the DPLUR off-diagonal blocks of implicitUpdateA (implicit.c:689-813; implicitUpdateA_sa
 // 860-935), one thread per interior face slot j of a cell: the finite-difference Jacobian (h = 1e-6) of the
-// neighbour's face flux, minus half the face's spectral radius on the diagonal. A block needs only the
-// state at the start of the iteration (and, for SA, the face eddy viscosity of k_flux), so the engine runs
-// this kernel beside the gradient and flux kernels. Blocks [j gb, (j + 1) gb) of the grid hold slot j of
-// the cells of cell blocks [0, gb).
+// neighbour's face flux, minus half the face's spectral radius on the diagonal. A block needs only the state at the
+// start of the iteration and k_side's quantities, so the engine runs this kernel beside the gradient and flux kernels.
+// Blocks [j gb, (j + 1) gb) of the grid hold slot j of the cells of cell blocks [0, gb).
+//
+// Bound by FP64 issue and the latency of its gathers; most of it was divisions that k_side now does once per cell or
+// face (pressures, unit normals, spectral radii) or that over_h replaces. With k_side: SA plate 143 -> 84 us (its
+// diagonal 35 -> 15), 100,000-cell SA FP64 77 -> 52, 160,000 triangles 43 -> 42 (19 -> 12.5), 500,000 125 -> 123
+// (43 -> 23). Registers for three blocks per SM (SST two; four: SA the same, 500,000 triangles 133).
 // ------------------------------------------------------------------------------------------------
 template <int MODEL>
-__global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_blocks(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+__global__ void __launch_bounds__(BLOCK, MODEL == 2 ? 2 : 3) k_blocks(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
                                                   const __grid_constant__ State s, int gb, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
@@ -1156,68 +1261,42 @@ __global__ void __launch_bounds__(BLOCK, MODEL == 0 ? 3 : 2) k_blocks(const Prm*
     const int c = cb * BLOCK + threadIdx.x;
     if (!cell_in(p, c)) return;
     const int nc = m.nc;
+    const int sf = m.fslot[j * nc + c], nb = m.fnb[j * nc + c];
     if (j >= m.nint[c]) return;
-    const int sf = m.fslot[(size_t)j * nc + c];
     const int f = sf > 0 ? sf - 1 : -sf - 1;
-    const int2 e = m.fe[f];
-    const int nb = sf > 0 ? e.y : e.x;
-    const double2 dSv = m.fn[f];
-    const double dSx = sf > 0 ? dSv.x : -dSv.x, dSy = sf > 0 ? dSv.y : -dSv.y;
+    const double2 un = m.fun[f];
+    const double nx = sf > 0 ? un.x : -un.x, ny = sf > 0 ? un.y : -un.y;
     const double dS = m.fds[f];
-    const double nx = dSx / dS, ny = dSy / dS;
-    const double h = 1.0e-6;
-    double Un[NV], Pn[NP];
+    double Un[NV], Pn[NP], pr[NV];
     loadU<MODEL>(s, nc, nb, Un);
     loadP<MODEL>(s, nc, nb, Pn);
+    {
+        const double4 t = s.PR4[nb];
+        pr[0] = t.x; pr[1] = t.y; pr[2] = t.z; pr[3] = t.w;
+        if constexpr (MODEL == 2) pr[4] = s.PRx[nb];
+        // the last variable (nt, omega) is in no energy: e2Taprox returns the temperature itself
+        if constexpr (MODEL >= 1) pr[NV - 1] = p.gas.R * Un[0] * Pn[4];
+    }
     double F0[NV], F[NV], Uq[NV];
-    double rho = Un[0];
-    double uu = Un[1] / rho;
-    double vv = Un[2] / rho;
-    double E = Un[3] / rho;
     aux_flux<NV>(Un, Pn[3], nx, ny, F0);
-    double ee0 = E - 0.5 * (uu * uu + vv * vv);
-    // SST (an extension: the reference's SST DPLUR multiplies 4x4 blocks into six variables, implicit.c:
-    // 990-1000 with 938-972): the energy holds the turbulent kinetic energy, as in its SST delta flux
-    // (implicitCalcDeltaFlux_sst, implicit.c:1048-1118)
-    if constexpr (MODEL == 2) ee0 = ee0 - Un[4] / rho;
     double A[NV * NV];
 #pragma unroll
     for (int mm = 0; mm < NV; mm++) {
-        // SST: rho omega reaches 1e10 beside a wall, where a step of 1e-6 is below its last bit; its column
-        // (a flux linear in rho omega) takes a step relative to the value
-        const double hm = MODEL == 2 && mm >= 4 ? h * fmax(1.0, fabs(Un[mm])) : h;
+        const double hm = pert_step<MODEL>(mm, Un);
 #pragma unroll
         for (int nn = 0; nn < NV; nn++) Uq[nn] = mm == nn ? Un[nn] + hm : Un[nn];
-        double r2 = Uq[0];
-        double u2 = Uq[1] / r2;
-        double v2 = Uq[2] / r2;
-        double E2 = Uq[3] / r2;
-        double ee1 = E2 - 0.5 * (u2 * u2 + v2 * v2);
-        if constexpr (MODEL == 2) ee1 = ee1 - Uq[4] / r2;
-        double T = e2Taprox(p.gas, ee0, Pn[4], ee1);
-        double pr = p.gas.R * r2 * T;
-        aux_flux<NV>(Uq, pr, nx, ny, F);
+        aux_flux<NV>(Uq, pr[mm], nx, ny, F);
 #pragma unroll
-        for (int nn = 0; nn < NV; nn++) A[nn * NV + mm] = 0.5 * (F[nn] - F0[nn]) * dS / hm;
+        for (int nn = 0; nn < NV; nn++) {
+            if (!block_nz(nn, mm)) continue;
+            const double d = 0.5 * (F[nn] - F0[nn]) * dS;
+            A[nn * NV + mm] = MODEL == 2 && mm >= 4 ? d / hm : over_h(d);
+        }
     }
     double cc = T2c(p.gas, Pn[4]);
     double ra = p.w_imp * (fabs(nx * Pn[1] + ny * Pn[2]) + cc) * dS;
-    if constexpr (MODEL >= 1) {
-        // implicitUpdateA_sa (implicit.c:920-928): always viscous, with the face eddy viscosity (SST: the
-        // same radius with its own eddy viscosity)
-        double Pc[NP];
-        loadP<MODEL>(s, nc, c, Pc);
-        double r = (Pc[0] + Pn[0]) * 0.5;
-        double T = (Pc[4] + Pn[4]) * 0.5;
-        double mi = sutherland(T);
-        ra += fmax(4 / (3 * r), T2gamma(p.gas, T) / r) * (mi / p.pr + s.MIT[f] / p.pr_t) * dS / m.fL[f];
-    } else if (p.laminar) {
-        double Pc[NP];
-        loadP<MODEL>(s, nc, c, Pc);
-        double r = (Pc[0] + Pn[0]) * 0.5;
-        double T = (Pc[4] + Pn[4]) * 0.5;
-        ra += visc_radius(p.gas, p.pr, r, T) * dS / m.fL[f];
-    }
+    // implicitUpdateA_sa (implicit.c:920-928): with the face eddy viscosity (SST: the same radius with its own)
+    if (MODEL >= 1 || p.laminar) ra += s.FB[f];
 #pragma unroll
     for (int nn = 0; nn < NV; nn++) A[nn * NV + nn] -= 0.5 * ra;
     const size_t base = block_at<MODEL>(c, j, slots);
@@ -1557,10 +1636,9 @@ __global__ void __launch_bounds__(LUSGS_THREADS) k_lusgs(const Prm* __restrict__
     for (int k = 0; k < NV; k++) term[k] = 0.0;
     if (mine && store) {
         const int f = sf > 0 ? sf - 1 : -sf - 1;
-        double2 dSv = m.fn[f];
-        double dSx = sf > 0 ? dSv.x : -dSv.x, dSy = sf > 0 ? dSv.y : -dSv.y;
+        double2 un = m.fun[f];
+        double nx = sf > 0 ? un.x : -un.x, ny = sf > 0 ? un.y : -un.y;
         double dS = m.fds[f];
-        double nx = dSx / dS, ny = dSy / dS;
         double Pn[NP], dn[NV], dF[NV];
         loadP<MODEL>(s, nc, nb, Pn);
         {

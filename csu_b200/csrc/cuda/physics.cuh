@@ -16,6 +16,7 @@ __device__ __constant__ static const double TP_CC[6] = {1.81716e3, 9.890504e2 - 
 
 struct Gas {
     double gamma, R, Cp, Cv;
+    double gam, gamR; // calorically perfect: (Cv + R) / Cv and that times R, divided once instead of per call
     int tp;
 };
 
@@ -83,13 +84,14 @@ __device__ __forceinline__ double e2T(const Gas& g, double e)
 // gasprop_T2gamma (gasprop.c:150-154) and gasprop_T2c (138-141)
 __device__ __forceinline__ double T2gamma(const Gas& g, double T)
 {
+    if (!g.tp) return g.gam;
     double Cv = T2Cv(g, T);
     return (Cv + g.R) / Cv;
 }
 
 __device__ __forceinline__ double T2c(const Gas& g, double T)
 {
-    return sqrt(T2gamma(g, T) * g.R * T);
+    return sqrt((g.tp ? T2gamma(g, T) * g.R : g.gamR) * T);
 }
 
 // gasprop_e2Taprox (gasprop.c:156-159)
