@@ -241,9 +241,6 @@ static void plan(csu_ctx* x, Arena& a)
     m.nei = carve<int>(a, c4);
     m.lw = carve<double2>(a, c4);
     m.ld = carve<double2>(a, c4);
-    m.lm = carve<unsigned long long>(a, c4);
-    m.les = carve<int>(a, c4);
-    m.lrv = carve<unsigned long long>(a, nc);
     m.lq = carve<double2>(a, c4);
     m.lk = carve<double2>(a, (size_t)3 * nc);
     m.lim3 = carve<double>(a, nc);
@@ -251,10 +248,12 @@ static void plan(csu_ctx* x, Arena& a)
     m.fslot = carve<int>(a, c4);
     m.fnb = carve<int>(a, c4);
     m.omega = carve<double>(a, nc);
-    m.sxh = carve<double>(a, nc);
-    m.syh = carve<double>(a, nc);
+    // local steps of the explicit schemes only
+    const bool rk = x->cfg.time_scheme == CSU_TS_RK;
+    m.sxh = rk ? carve<double>(a, nc) : nullptr;
+    m.syh = rk ? carve<double>(a, nc) : nullptr;
     m.wall_d = (x->is_pack ? x->pack_wall_d : x->L.wall_d != nullptr) ? carve<double>(a, nc) : nullptr;
-    m.dslat = carve<double>(a, nc);
+    m.dslat = x->cfg.axisymmetric ? carve<double>(a, nc) : nullptr;
     m.fe = carve<int2>(a, nf);
     m.fn = carve<double2>(a, nf);
     m.fun = carve<double2>(a, nf);
@@ -272,8 +271,9 @@ static void plan(csu_ctx* x, Arena& a)
     m.bL = carve<double>(a, nb);
     m.bun = carve<double2>(a, nb);
     m.bds2 = carve<double>(a, nb);
-    m.color = carve<int>(a, nc);
-    m.color_cells = carve<int>(a, nc);
+    const bool lusgs = x->cfg.time_scheme == CSU_TS_LUSGS;
+    m.color = lusgs ? carve<int>(a, nc) : nullptr;
+    m.color_cells = lusgs ? carve<int>(a, nc) : nullptr;
     x->d_wall_rank = carve<int>(a, nb);
 
     s.U4 = carve<double4>(a, nc);
@@ -391,9 +391,6 @@ static int upload_mesh(csu_ctx* x)
     CK(up(m.nei, L.nei, sizeof(int) * c4));
     CK(up(m.lw, L.lw, sizeof(double2) * c4));
     CK(up(m.ld, L.ld, sizeof(double2) * c4));
-    CK(up(m.lm, L.lm, sizeof(unsigned long long) * c4));
-    CK(up(m.les, L.les, sizeof(int) * c4));
-    CK(up(m.lrv, L.lrv, sizeof(unsigned long long) * nc));
     CK(up(m.lq, L.lq, sizeof(double2) * c4));
     CK(up(m.lk, L.lk, sizeof(double2) * 3 * nc));
     CK(up(m.em, L.em, sizeof(double2) * c4));
@@ -401,10 +398,10 @@ static int upload_mesh(csu_ctx* x)
     CK(up(m.fnb, L.fnb, sizeof(int) * c4));
     CK(up(x->d_n2o, L.cell_new2old, sizeof(int) * nc));
     CK(up(m.omega, L.omega, sizeof(double) * nc));
-    CK(up(m.sxh, L.sxh, sizeof(double) * nc));
-    CK(up(m.syh, L.syh, sizeof(double) * nc));
+    if (m.sxh) CK(up(m.sxh, L.sxh, sizeof(double) * nc));
+    if (m.syh) CK(up(m.syh, L.syh, sizeof(double) * nc));
     if (m.wall_d) CK(up(m.wall_d, L.wall_d, sizeof(double) * nc));
-    CK(up(m.dslat, L.dslat, sizeof(double) * nc));
+    if (m.dslat) CK(up(m.dslat, L.dslat, sizeof(double) * nc));
     CK(up(m.fe, fe.data(), sizeof(int2) * nf));
     CK(up(m.fn, fn.data(), sizeof(double2) * nf));
     CK(up(m.fun, fun.data(), sizeof(double2) * nf));
@@ -422,8 +419,8 @@ static int upload_mesh(csu_ctx* x)
     CK(up(m.bL, L.bL, sizeof(double) * nb));
     CK(up(m.bun, bun.data(), sizeof(double2) * nb));
     CK(up(m.bds2, L.bds2, sizeof(double) * nb));
-    CK(up(m.color, L.color, sizeof(int) * nc));
-    CK(up(m.color_cells, L.color_cells, sizeof(int) * nc));
+    if (m.color) CK(up(m.color, L.color, sizeof(int) * nc));
+    if (m.color_cells) CK(up(m.color_cells, L.color_cells, sizeof(int) * nc));
     CK(up(x->d_wall_rank, rank.data(), sizeof(int) * nb));
     return CSU_OK;
 }
@@ -2047,8 +2044,10 @@ extern "C" int csu_prep_create(const csu_mesh_desc* md, const csu_config* cfg, c
         csu_set_error("csu_prep_create: mesh layout failed (a cell with more than four faces?)");
         return st;
     }
-    // device bytes of the solve: the arena a one-solve context would carve, plus 1024 history rows
+    // device bytes of the solve: what a pack would carve for it alone, plus 1024 history rows
     csu_ctx t;
+    t.is_pack = true;
+    t.pack_wall_d = p->L.wall_d != nullptr;
     t.model = model;
     t.nv = nv;
     t.cfg = *cfg;
@@ -2226,16 +2225,19 @@ static std::vector<SegArr> seg_arrays(csu_ctx* x)
     auto P = [](const void* p) { return (char*)const_cast<void*>(p); };
     std::vector<SegArr> v = {
         {P(m.npts), 4, SEG_CELL}, {P(m.nint), 4, SEG_CELL}, {P(m.nslot), 4, SEG_CELL},
-        {P(m.nei), 4, SEG_CELL4}, {P(m.lw), 16, SEG_CELL4}, {P(m.ld), 16, SEG_CELL4}, {P(m.lm), 8, SEG_CELL4},
-        {P(m.les), 4, SEG_CELL4}, {P(m.lrv), 8, SEG_CELL}, {P(m.lq), 16, SEG_CELL4},
+        {P(m.nei), 4, SEG_CELL4}, {P(m.lw), 16, SEG_CELL4}, {P(m.ld), 16, SEG_CELL4}, {P(m.lq), 16, SEG_CELL4},
         {P(m.lk), 16, SEG_CELL3}, {P(m.em), 16, SEG_CELL4}, {P(m.fslot), 4, SEG_CELL4}, {P(m.fnb), 4, SEG_CELL4},
-        {P(m.omega), 8, SEG_CELL}, {P(m.sxh), 8, SEG_CELL}, {P(m.syh), 8, SEG_CELL},
-        {P(m.dslat), 8, SEG_CELL}, {P(m.color), 4, SEG_CELL},
+        {P(m.omega), 8, SEG_CELL},
         {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fun), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE}, {P(m.r0), 16, SEG_FACE},
         {P(m.r1), 16, SEG_FACE}, {P(m.fd), 16, SEG_FACE}, {P(m.fL), 8, SEG_FACE},
         {P(m.bown), 4, SEG_BFACE}, {P(m.bflag), 4, SEG_BFACE}, {P(m.bold), 4, SEG_BFACE},
         {P(m.bn), 16, SEG_BFACE}, {P(m.bds), 8, SEG_BFACE}, {P(m.bd), 16, SEG_BFACE}, {P(m.bL), 8, SEG_BFACE},
         {P(m.bun), 16, SEG_BFACE}, {P(m.bds2), 8, SEG_BFACE}, {P(x->d_wall_rank), 4, SEG_BFACE}};
+    // the rows only some settings have, as seg_host
+    if (m.sxh) v.push_back({P(m.sxh), 8, SEG_CELL});
+    if (m.syh) v.push_back({P(m.syh), 8, SEG_CELL});
+    if (m.dslat) v.push_back({P(m.dslat), 8, SEG_CELL});
+    if (m.color) v.push_back({P(m.color), 4, SEG_CELL});
     if (m.wall_d) v.push_back({P(m.wall_d), 8, SEG_CELL});
     return v;
 }
@@ -2255,7 +2257,7 @@ static int local_wall_ranks(const csu_layout& L, int* rank)
 }
 
 // The same arrays of one solve's host layout, in seg_arrays order (device formats built in `keep`).
-static std::vector<const void*> seg_host(const csu_layout& L, std::vector<std::vector<char>>& keep)
+static std::vector<const void*> seg_host(const Mesh& m, const csu_layout& L, std::vector<std::vector<char>>& keep)
 {
     const int nf = L.nf, nb = L.nb;
     auto pairs = [&](const double* a, const double* b, int n) {
@@ -2277,12 +2279,15 @@ static std::vector<const void*> seg_host(const csu_layout& L, std::vector<std::v
     int* rank = (int*)keep.back().data();
     local_wall_ranks(L, rank);
     std::vector<const void*> v = {
-        L.npts, L.nint, L.nslot, L.nei, L.lw, L.ld, L.lm, L.les, L.lrv, L.lq, L.lk, L.em, L.fslot, L.fnb,
-        L.omega, L.sxh, L.syh, L.dslat, L.color,
+        L.npts, L.nint, L.nslot, L.nei, L.lw, L.ld, L.lq, L.lk, L.em, L.fslot, L.fnb, L.omega,
         fe, pairs(L.fdsx, L.fdsy, nf), unit(), L.fds, pairs(L.r0x, L.r0y, nf), pairs(L.r1x, L.r1y, nf),
         pairs(L.fdx, L.fdy, nf), L.fdist,
         L.bown, L.bflag, L.bold, pairs(L.bdsx, L.bdsy, nb), L.bds, pairs(L.bdx, L.bdy, nb), L.bL,
         pairs(L.bunx, L.buny, nb), L.bds2, rank};
+    if (m.sxh) v.push_back(L.sxh);
+    if (m.syh) v.push_back(L.syh);
+    if (m.dslat) v.push_back(L.dslat);
+    if (m.color) v.push_back(L.color);
     if (L.wall_d) v.push_back(L.wall_d);
     return v;
 }
@@ -2490,7 +2495,7 @@ static int seg_fill(csu_ctx* x, int k, const csu_layout* L, csu_ctx* src, int ks
     } else {
         S = {0, L->nc, 0, L->nf, 0, L->nb, L->nc, L->nf, 0};
         std::vector<std::vector<char>> keep;
-        std::vector<const void*> from = seg_host(*L, keep);
+        std::vector<const void*> from = seg_host(x->mesh, *L, keep);
         if (from.size() != dst.size()) return CSU_ERR_INPUT;
         CK(cudaStreamSynchronize(x->stream));
         for (size_t a = 0; a < dst.size(); a++) {
@@ -2629,7 +2634,7 @@ static int pack_build(const char* who, const csu_prep* const* solves, int n, csu
         cudaError_t e = cudaStreamSynchronize(x->stream);
         if (e == cudaSuccess && n > 1) e = cudaMemcpy(const_cast<int*>(x->st.bsolve), bs.data(), sizeof(int) * nblk, cudaMemcpyHostToDevice);
         if (e == cudaSuccess && n > 1) e = cudaMemcpy(const_cast<int*>(x->st.csolve), cs.data(), sizeof(int) * NC, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && x->mesh.color_cells)
             e = cudaMemcpy(const_cast<int*>(x->mesh.color_cells), color_cells.data(), sizeof(int) * NC,
                            cudaMemcpyHostToDevice);
         if (e != cudaSuccess) st = cuda_fail(e, "pack maps");

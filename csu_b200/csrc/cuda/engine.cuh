@@ -117,9 +117,6 @@ struct Mesh {
     const double2* lw;              // [4][nc] gradient weights (LSQ 0)
     const double2* em;              // [4][nc] edge midpoint minus centroid
     const double2* ld;              // [4][nc] least squares: neighbour centre minus centroid
-    const unsigned long long* lm;   // [4][nc] x87 significands of a, b, c, det
-    const int* les;                 // [4][nc] exponent << 1 | sign
-    const unsigned long long* lrv;  // reciprocal of det's significand
     const double2* lq;              // [4][nc] a, b, c and 1/det as exact (h, l) double-doubles
     const double2* lk;              // [3][nc] a, b, c over det as (h, l) double-doubles
     const double* lim3;             // (K sqrt(omega / omega_max))^3 of the limiter's epsilon^2 (k_lim3)

@@ -105,18 +105,6 @@ __global__ void __launch_bounds__(BLOCK) k_prim(const Prm* __restrict__ P, const
 // ------------------------------------------------------------------------------------------------
 constexpr int GRAD_CELLS = 32;
 
-// x87 constants a, b, c, det of cell c (solver.c:1063-1073, evaluated on the host in long double)
-__device__ __forceinline__ void lsq_consts(const Mesh& m, int nc, int c, X80* K)
-{
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        int es = m.les[(size_t)q * nc + c];
-        K[q].m = m.lm[(size_t)q * nc + c];
-        K[q].e = es >> 1;
-        K[q].s = es & 1;
-    }
-}
-
 // k_lim3: the cell-size factor of limiterCalc's epsilon^2, type 0 (limiter.c:98-119), which no iteration changes.
 __global__ void __launch_bounds__(BLOCK) k_lim3(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
                                                 const __grid_constant__ State s, double* lim3)
@@ -178,12 +166,18 @@ __device__ __noinline__ double lsq_slot_x87(const Prm& p, const Mesh& m, const S
         X = x80_add(X, x80_from_double((y ? d.y : d.x) * du));
         Y = x80_add(Y, x80_from_double((y ? d.x : d.y) * du));
     }
-    X80 K[4];
-    lsq_consts(m, nc, c, K);
+    // a, b, c (exact as double-doubles) and det = a c - b b, rounded as the host's long double (solver.c:1063-1073)
+    X80 K[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const double2 v = m.lq[q * nc + c];
+        K[q] = x80_add(x80_from_double(v.x), x80_from_double(v.y));
+    }
+    const X80 det = x80_add(x80_mul(K[0], K[2]), x80_neg(x80_mul(K[1], K[1])));
     // (c A - b B) / det, (-b A + a B) / det: A + B and B + A round alike
     const X80 N = x80_add(x80_mul(y ? K[0] : K[2], X), x80_mul(x80_neg(K[1]), Y));
     atomicAdd(s.lsq_x87, 1ULL);
-    return x80_to_double(x80_div_pre(N, K[3], m.lrv[c]));
+    return x80_to_double(x80_div(N, det));
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -73,28 +73,6 @@ static unsigned long long hilbert_key(unsigned x, unsigned y)
     return d;
 }
 
-/* x87 long double as significand (bit 63 set) and exponent<<1|sign, the device's ext80 format */
-static void split_ld(long double v, unsigned long long* m, int* es)
-{
-    if (v == 0) {
-        *m = 0;
-        *es = signbit(v) ? 1 : 0;
-        return;
-    }
-    int e;
-    long double f = frexpl(fabsl(v), &e);
-    *m = (unsigned long long)ldexpl(f, 64);
-    *es = ((e - 64) * 2) | (v < 0 ? 1 : 0);
-}
-
-/* floor((2^128 - 1) / d) - 2^64 for a normalised d (invariant-divisor reciprocal) */
-static unsigned long long recip64(unsigned long long d)
-{
-    if (d == 0) return 0;
-    unsigned __int128 all = ~(unsigned __int128)0;
-    return (unsigned long long)(all / d - ((unsigned __int128)1 << 64));
-}
-
 typedef struct {
     unsigned long long key;
     int id;
@@ -114,7 +92,7 @@ void csu_layout_free(csu_layout* L)
                     L->bface_old2new, L->npts, L->nint, L->nslot, L->nei, L->lw, L->em,
                     L->fslot, L->fnb, L->omega, L->sxh, L->syh, L->xc, L->yc, L->wall_d, L->dslat, L->fe0, L->fe1,
                     L->fdsx, L->fdsy, L->fds, L->r0x, L->r0y, L->r1x, L->r1y, L->fdist, L->bown, L->bflag,
-                    L->bold, L->bdsx, L->bdsy, L->bds, L->bmx, L->bmy, L->ld, L->lm, L->les, L->lrv, L->lq, L->lk,
+                    L->bold, L->bdsx, L->bdsy, L->bds, L->bmx, L->bmy, L->ld, L->lq, L->lk,
                     L->fdx, L->fdy, L->bdx, L->bdy, L->bL, L->bunx, L->buny, L->bds2, L->color,
                     L->color_start, L->color_cells};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) free(ptrs[i]);
@@ -158,7 +136,7 @@ int csu_layout_build(const csu_mesh_desc* m, int axi, csu_layout* L)
     ALLOC(L->bface_new2old, nb); ALLOC(L->bface_old2new, nb);
     ALLOC(L->npts, nc); ALLOC(L->nint, nc); ALLOC(L->nslot, nc); ALLOC(L->nei, c4);
     ALLOC(L->lw, 2 * c4); ALLOC(L->em, 2 * c4); ALLOC(L->fslot, c4); ALLOC(L->fnb, c4);
-    ALLOC(L->ld, 2 * c4); ALLOC(L->lm, c4); ALLOC(L->les, c4); ALLOC(L->lrv, nc); ALLOC(L->lq, 2 * c4);
+    ALLOC(L->ld, 2 * c4); ALLOC(L->lq, 2 * c4);
     ALLOC(L->lk, (size_t)6 * nc);
     ALLOC(L->omega, nc); ALLOC(L->sxh, nc); ALLOC(L->syh, nc); ALLOC(L->xc, nc); ALLOC(L->yc, nc);
     ALLOC(L->dslat, nc);
@@ -347,11 +325,9 @@ int csu_layout_build(const csu_mesh_desc* m, int axi, csu_layout* L)
             cc += dy[j] * dy[j];
         }
         long double det = a * cc - bb * bb;
-        long double k4[4] = {a, bb, cc, det};
-        for (int q = 0; q < 4; q++) split_ld(k4[q], &L->lm[(size_t)q * nc + c], &L->les[(size_t)q * nc + c]);
-        L->lrv[c] = recip64(L->lm[(size_t)3 * nc + c]);
-        /* the same as exact double-doubles for the device's certified FP64 evaluation: a, b, c as
-           (RN53, remainder) and 1/det to ~2^-103 (FP64 reciprocal + one Newton correction) */
+        long double k4[3] = {a, bb, cc};
+        /* as exact double-doubles for the device's certified FP64 evaluation: a, b, c as (RN53, remainder) and
+           1/det to ~2^-103 (FP64 reciprocal + one Newton correction) */
         for (int q = 0; q < 3; q++) {
             double h = (double)k4[q];
             L->lq[2 * ((size_t)q * nc + c)] = h;

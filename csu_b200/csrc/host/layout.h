@@ -30,9 +30,6 @@ typedef struct csu_layout {
     int* nei;      /* [4][nc] neighbour (ELEMENT.neiL order): cell id, or nc + boundary face id       */
     double* lw;    /* [4][nc][2] least-squares weights: dUx = sum wx (u_nei - u_cell), dUy with wy       */
     double* ld;    /* [4][nc][2] neighbour centre minus centroid (solverCalcGrad3 x[jj] - x[0])          */
-    unsigned long long* lm;  /* [4][nc] x87 significands of a, b, c, a*c - b*b (long double, solver.c:1058-1073) */
-    int* les;      /* [4][nc] exponent << 1 | sign of the same                                          */
-    unsigned long long* lrv; /* [nc] invariant-divisor reciprocal of the determinant's significand       */
     double* lq;    /* [4][nc][2] a, b, c, 1/(a*c - b*b) as (high, low) double pairs                          */
     double* lk;    /* [3][nc][2] a, b, c over (a*c - b*b) as (high, low) double pairs                        */
     double* em;    /* [4][nc][2] edge midpoint minus centroid, edges in node order (limiter, inter)     */
