@@ -219,10 +219,24 @@ __device__ __forceinline__ double ordbits_inv(unsigned long long b)
     return bitsd((b & 0x8000000000000000ULL) ? (b & 0x7fffffffffffffffULL) : ~b);
 }
 
+// A 32-byte record as one access (sm_100's 256-bit loads and stores; double4 arrays are 256-byte aligned): half the
+// requests of the two 16-byte ones the compiler makes of a double4, which random gathers pay for one by one.
+__device__ __forceinline__ double4 ld4(const double4* p)
+{
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ void st4(double4* p, double4 v)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+
 template <int MODEL>
 __device__ __forceinline__ void loadU(const State& s, int nc, int i, double* q)
 {
-    double4 t = s.U4[i];
+    double4 t = ld4(s.U4 + i);
     q[0] = t.x; q[1] = t.y; q[2] = t.z; q[3] = t.w;
 #pragma unroll
     for (int k = 4; k < Model<MODEL>::NV; k++) q[k] = s.Ux[(size_t)(k - 4) * nc + i];
@@ -231,7 +245,7 @@ __device__ __forceinline__ void loadU(const State& s, int nc, int i, double* q)
 template <int MODEL>
 __device__ __forceinline__ void storeU(const State& s, int nc, int i, const double* q)
 {
-    s.U4[i] = make_double4(q[0], q[1], q[2], q[3]);
+    st4(s.U4 + i, make_double4(q[0], q[1], q[2], q[3]));
 #pragma unroll
     for (int k = 4; k < Model<MODEL>::NV; k++) s.Ux[(size_t)(k - 4) * nc + i] = q[k];
 }
@@ -240,7 +254,7 @@ __device__ __forceinline__ void storeU(const State& s, int nc, int i, const doub
 template <int MODEL>
 __device__ __forceinline__ void loadP(const State& s, int nc, int i, double* P)
 {
-    double4 t = s.W4[i];
+    double4 t = ld4(s.W4 + i);
     P[0] = t.x; P[1] = t.y; P[2] = t.z; P[3] = t.w;
     P[4] = s.WT[i];
 #pragma unroll
@@ -250,7 +264,7 @@ __device__ __forceinline__ void loadP(const State& s, int nc, int i, double* P)
 template <int MODEL>
 __device__ __forceinline__ void storeP(const State& s, int nc, int i, const double* P)
 {
-    s.W4[i] = make_double4(P[0], P[1], P[2], P[3]);
+    st4(s.W4 + i, make_double4(P[0], P[1], P[2], P[3]));
     s.WT[i] = P[4];
 #pragma unroll
     for (int k = 5; k < Model<MODEL>::NP; k++) s.Wx[(size_t)(k - 5) * nc + i] = P[k];

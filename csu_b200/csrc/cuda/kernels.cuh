@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), grad_bloc
 template <int MODEL>
 __device__ __forceinline__ void owner_visc_gradients(const State& s, int nc, int c, double* gvx, double* gvy)
 {
-    double4 a = s.G4x[c], bb = s.G4y[c];
+    double4 a = ld4(s.G4x + c), bb = ld4(s.G4y + c);
     gvx[0] = a.y; gvx[1] = a.z; gvx[2] = s.GTx[c];
     gvy[0] = bb.y; gvy[1] = bb.z; gvy[2] = s.GTy[c];
     gvx[3] = MODEL >= 1 ? s.Gxx[c] : 0.0;
@@ -456,7 +456,7 @@ __device__ __forceinline__ void bface_visc(const Prm& p, const Mesh& m, const St
         double fv[5];
         sst_boundary_flux(p.gas, p.sst_k, p.pr, p.pr_t, p.t_wall, p.pin, flag, gvx, gvy, E0, m.wall_d[c], dSx, dSy,
                           bdv.x, bdv.y, bLv, un.x, un.y, m.bds2[b], fv);
-        s.FV[fi] = make_double4(fv[0], fv[1], fv[2], fv[3]);
+        st4(s.FV + fi, make_double4(fv[0], fv[1], fv[2], fv[3]));
         s.FV5[fi] = fv[4];
     } else if constexpr (MODEL == 1) {
         double2 un = m.bun[b];
@@ -467,14 +467,14 @@ __device__ __forceinline__ void bface_visc(const Prm& p, const Mesh& m, const St
         else
             sa_boundary_flux(p.gas, p.pr, p.pr_t, p.t_wall, p.pin, flag, gvx, gvy, E0, dSx, dSy, bdv.x, bdv.y, bLv,
                              un.x, un.y, m.bds2[b], fv);
-        s.FV[fi] = make_double4(fv[0], fv[1], fv[2], fv[3]);
+        st4(s.FV + fi, make_double4(fv[0], fv[1], fv[2], fv[3]));
     } else {
         if (p.laminar == 1) {
             double2 un = m.bun[b];
             double fv[3];
             laminar_boundary(p.gas, p.pr, p.t_wall, p.pin, flag, gvx, gvy, E0, dSx, dSy, bdv.x, bdv.y, bLv, un.x,
                              un.y, m.bds2[b], fv);
-            s.FV[fi] = make_double4(fv[0], fv[1], fv[2], 0.0);
+            st4(s.FV + fi, make_double4(fv[0], fv[1], fv[2], 0.0));
         }
     }
 }
@@ -572,7 +572,7 @@ __device__ __forceinline__ void interior_face(const Prm& p, const Mesh& m, const
         double fv[5], mit;
         sst_face_flux(p.gas, p.sst_k, p.pr, p.pr_t, g0x, g0y, g1x, g1y, A, B, m.wall_d[e.x], m.wall_d[e.y], dd.x,
                       dd.y, m.fL[f], dSx, dSy, fv, &mit);
-        s.FV[f] = make_double4(fv[0], fv[1], fv[2], fv[3]);
+        st4(s.FV + f, make_double4(fv[0], fv[1], fv[2], fv[3]));
         s.FV5[f] = fv[4];
         s.MIT[f] = mit;
     } else if constexpr (MODEL == 1) {
@@ -586,7 +586,7 @@ __device__ __forceinline__ void interior_face(const Prm& p, const Mesh& m, const
         else
             sa_face_flux(p.gas, p.pr, p.pr_t, p.visc_blazek, g0x, g0y, g1x, g1y, A, B, dd.x, dd.y, m.fL[f], dSx,
                          dSy, fv, &mit);
-        s.FV[f] = make_double4(fv[0], fv[1], fv[2], fv[3]);
+        st4(s.FV + f, make_double4(fv[0], fv[1], fv[2], fv[3]));
         if (!p.mit_early) s.MIT[f] = mit;
     } else if (p.laminar == 1) {
         const double4 a = gx0, b = gy0, cc = gx1, d = gy1;
@@ -595,14 +595,14 @@ __device__ __forceinline__ void interior_face(const Prm& p, const Mesh& m, const
         double2 dd = m.fd[f];
         double fv[3];
         laminar_face(p.gas, p.pr, g0x, g0y, g1x, g1y, A, B, dd.x, dd.y, m.fL[f], dSx, dSy, fv);
-        s.FV[f] = make_double4(fv[0], fv[1], fv[2], 0.0);
+        st4(s.FV + f, make_double4(fv[0], fv[1], fv[2], 0.0));
     }
     rotation(PL, dSx, dSy, dS);
     rotation(PR, dSx, dSy, dS);
     double fl[NV];
     riemann<MODEL>(p.scheme, p.gas, p.e_fix, p.mach_inf, PL, PR, fl);
     rotation(fl, dSx, -dSy, dS);
-    s.F4[f] = make_double4(fl[0] * dS, fl[1] * dS, fl[2] * dS, fl[3] * dS);
+    st4(s.F4 + f, make_double4(fl[0] * dS, fl[1] * dS, fl[2] * dS, fl[3] * dS));
 #pragma unroll
     for (int kk = 4; kk < NV; kk++) s.Fx[(size_t)(kk - 4) * (m.nf + m.nb) + f] = fl[kk] * dS;
 }
@@ -629,8 +629,8 @@ __device__ __forceinline__ void boundary_face(const Prm* __restrict__ P, const M
     boundary_flux<MODEL>(p, flag, dSx, dSy, dS, E0, fl);
     int fi = m.nf + b;
     double sc = dS > 0 ? dS : 0.0;
-    s.F4[fi] = dS > 0 ? make_double4(fl[0] * dS, fl[1] * dS, fl[2] * dS, fl[3] * dS)
-                      : make_double4(0.0, 0.0, 0.0, 0.0);
+    st4(s.F4 + fi, dS > 0 ? make_double4(fl[0] * dS, fl[1] * dS, fl[2] * dS, fl[3] * dS)
+                          : make_double4(0.0, 0.0, 0.0, 0.0));
 #pragma unroll
     for (int kk = 4; kk < NV; kk++) s.Fx[(size_t)(kk - 4) * (m.nf + m.nb) + fi] = dS > 0 ? fl[kk] * sc : 0.0;
     double gvx[5], gvy[5];
@@ -682,9 +682,9 @@ __global__ void __launch_bounds__(FB) k_flux(const Prm* __restrict__ P, const __
         pdl_wait();
         if (halted_behind(p, s.sc + sid)) return;
         const double4 z4 = make_double4(0.0, 0.0, 0.0, 0.0);
-        interior_face<MODEL>(p, m, s, f, e, s.W4[e.x], s.WT[e.x], grad ? s.G4x[e.x] : z4, grad ? s.G4y[e.x] : z4,
-                             o2 ? s.PH4[e.x] : z4, s.W4[e.y], s.WT[e.y], grad ? s.G4x[e.y] : z4,
-                             grad ? s.G4y[e.y] : z4, o2 ? s.PH4[e.y] : z4);
+        interior_face<MODEL>(p, m, s, f, e, ld4(s.W4 + e.x), s.WT[e.x], grad ? ld4(s.G4x + e.x) : z4,
+                             grad ? ld4(s.G4y + e.x) : z4, o2 ? ld4(s.PH4 + e.x) : z4, ld4(s.W4 + e.y), s.WT[e.y],
+                             grad ? ld4(s.G4x + e.y) : z4, grad ? ld4(s.G4y + e.y) : z4, o2 ? ld4(s.PH4 + e.y) : z4);
     } else {
         int b = (blockIdx.x - nbi) * FB + threadIdx.x;
         if (b >= m.nb) return;
@@ -724,13 +724,13 @@ __global__ void __launch_bounds__(FB) k_flux_st(const Prm* __restrict__ P, const
     for (int i = threadIdx.x; i < WIN; i += FB) {
         const int c = base + i;
         if (c < nc) {
-            sw[i] = s.W4[c];
+            sw[i] = ld4(s.W4 + c);
             st[i] = s.WT[c];
             if (grad) {
-                sgx[i] = s.G4x[c];
-                sgy[i] = s.G4y[c];
+                sgx[i] = ld4(s.G4x + c);
+                sgy[i] = ld4(s.G4y + c);
             }
-            if (o2) sph[i] = s.PH4[c];
+            if (o2) sph[i] = ld4(s.PH4 + c);
         }
     }
     __syncthreads();
@@ -742,18 +742,18 @@ __global__ void __launch_bounds__(FB) k_flux_st(const Prm* __restrict__ P, const
     const double4 z4 = make_double4(0.0, 0.0, 0.0, 0.0);
     const unsigned i0 = (unsigned)(e.x - base), i1 = (unsigned)(e.y - base);
     const bool in0 = i0 < (unsigned)WIN, in1 = i1 < (unsigned)WIN;
-    const double4 w0 = in0 ? sw[i0] : s.W4[e.x], w1 = in1 ? sw[i1] : s.W4[e.y];
+    const double4 w0 = in0 ? sw[i0] : ld4(s.W4 + e.x), w1 = in1 ? sw[i1] : ld4(s.W4 + e.y);
     const double t0 = in0 ? st[i0] : s.WT[e.x], t1 = in1 ? st[i1] : s.WT[e.y];
     double4 gx0 = z4, gy0 = z4, gx1 = z4, gy1 = z4, ph0 = z4, ph1 = z4;
     if (grad) {
-        gx0 = in0 ? sgx[i0] : s.G4x[e.x];
-        gy0 = in0 ? sgy[i0] : s.G4y[e.x];
-        gx1 = in1 ? sgx[i1] : s.G4x[e.y];
-        gy1 = in1 ? sgy[i1] : s.G4y[e.y];
+        gx0 = in0 ? sgx[i0] : ld4(s.G4x + e.x);
+        gy0 = in0 ? sgy[i0] : ld4(s.G4y + e.x);
+        gx1 = in1 ? sgx[i1] : ld4(s.G4x + e.y);
+        gy1 = in1 ? sgy[i1] : ld4(s.G4y + e.y);
     }
     if (o2) {
-        ph0 = in0 ? sph[i0] : s.PH4[e.x];
-        ph1 = in1 ? sph[i1] : s.PH4[e.y];
+        ph0 = in0 ? sph[i0] : ld4(s.PH4 + e.x);
+        ph1 = in1 ? sph[i1] : ld4(s.PH4 + e.y);
     }
     interior_face<MODEL>(p, m, s, f, e, w0, t0, gx0, gy0, ph0, w1, t1, gx1, gy1, ph1);
 }
@@ -774,7 +774,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
         if (j < ns) {
             int sf = m.fslot[(size_t)j * nc + c];
             int fi = sf > 0 ? sf - 1 : -sf - 1;
-            double4 F = s.F4[fi];
+            double4 F = ld4(s.F4 + fi);
             double fv[NV];
             fv[0] = F.x; fv[1] = F.y; fv[2] = F.z; fv[3] = F.w;
 #pragma unroll
@@ -802,7 +802,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
             if (j < ni) {
                 int sf = m.fslot[(size_t)j * nc + c];
                 int fi = sf > 0 ? sf - 1 : -sf - 1;
-                double4 V = s.FV[fi];
+                double4 V = ld4(s.FV + fi);
                 if (sf > 0) {
                     R[1] -= V.x;
                     R[2] -= V.y;
@@ -819,7 +819,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
             }
         }
         if constexpr (MODEL == 1) {
-            double4 gx = s.G4x[c], gy = s.G4y[c];
+            double4 gx = ld4(s.G4x + c), gy = ld4(s.G4y + c);
             double rho = P[0], T = P[4], n = P[5];
             double d = m.wall_d[c];
             double mi_L = sutherland(T);
@@ -830,7 +830,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
             R[4] -= Qt * m.omega[c];
         }
         if constexpr (MODEL == 2) {
-            double4 gx = s.G4x[c], gy = s.G4y[c];
+            double4 gx = ld4(s.G4x + c), gy = ld4(s.G4y + c);
             double sgx[4] = {gx.y, gx.z, s.Gxx[c], s.Gxx[(size_t)nc + c]};
             double sgy[4] = {gy.y, gy.z, s.Gxy[c], s.Gxy[(size_t)nc + c]};
             double Qtk, Qto;
@@ -844,7 +844,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
         for (int j = 0; j < 4; j++) {
             if (j >= ni && j < ns) {
                 int fi = m.fslot[(size_t)j * nc + c] - 1;
-                double4 V = s.FV[fi];
+                double4 V = ld4(s.FV + fi);
                 R[1] -= V.x;
                 R[2] -= V.y;
                 R[3] -= V.z;
@@ -858,7 +858,7 @@ __device__ __forceinline__ void gather_residual(const Prm& p, const Mesh& m, con
 template <int MODEL>
 __device__ __forceinline__ void storeR(const State& s, int nc, int c, const double* R)
 {
-    s.R4[c] = make_double4(R[0], R[1], R[2], R[3]);
+    st4(s.R4 + c, make_double4(R[0], R[1], R[2], R[3]));
 #pragma unroll
     for (int k = 4; k < Model<MODEL>::NV; k++) s.Rx[(size_t)(k - 4) * nc + c] = R[k];
 }
@@ -987,7 +987,7 @@ template <int MODEL>
 __device__ __forceinline__ void face_radii(const Prm& p, const Mesh& m, const State& s, int f, double* Lc, double* Lv)
 {
     const int2 e = m.fe[f];
-    const double4 w0 = s.W4[e.x], w1 = s.W4[e.y];
+    const double4 w0 = ld4(s.W4 + e.x), w1 = ld4(s.W4 + e.y);
     const double T0 = s.WT[e.x], T1 = s.WT[e.y];
     const double2 un = m.fun[f];
     const double dS = m.fds[f];
@@ -1040,7 +1040,7 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
                 // in nt (the gradients held), its negative (destruction-dominated) part taken implicitly:
                 // dQ = -Omega min(dQt/d(rho nt), 0) >= 0 joins the diagonal of the nt row
                 if (p.sa_isrc) {
-                    double4 gx = s.G4x[c], gy = s.G4y[c];
+                    double4 gx = ld4(s.G4x + c), gy = ld4(s.G4y + c);
                     double rho = P[0], T = P[4], n = P[5];
                     double d = m.wall_d[c];
                     double mi_L = sutherland(T);
@@ -1059,7 +1059,7 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
                 // the SST source Jacobians of the implicit diagonal (sstInterSource, sst.c:643-680): LU-SGS
                 // as the reference, DPLUR as the extension's k-omega diagonal block
                 if (s.dQ) {
-                    double4 gx = s.G4x[c], gy = s.G4y[c];
+                    double4 gx = ld4(s.G4x + c), gy = ld4(s.G4y + c);
                     double sgx[4] = {gx.y, gx.z, s.Gxx[c], s.Gxx[(size_t)nc + c]};
                     double sgy[4] = {gy.y, gy.z, s.Gxy[c], s.Gxy[(size_t)nc + c]};
                     double J[6];
@@ -1181,7 +1181,7 @@ __global__ void __launch_bounds__(BLOCK) k_side(const Prm* __restrict__ P, const
         const Prm& p = P[sid];
         if (halted(s.sc + sid)) return;
         if constexpr (MODEL == 1) {
-            const double r = (s.W4[e.y].x + s.W4[e.x].x) * 0.5;
+            const double r = (ld4(s.W4 + e.y).x + ld4(s.W4 + e.x).x) * 0.5;
             const double T = (s.WT[e.y] + s.WT[e.x]) * 0.5;
             const double n = (s.Wx[e.y] + s.Wx[e.x]) * 0.5;
             const double mi_L = sutherland(T);
@@ -1226,7 +1226,7 @@ __global__ void __launch_bounds__(BLOCK) k_side(const Prm* __restrict__ P, const
         double T = e2Taprox(p.gas, ee0, T0, ee1);
         pr[mm] = p.gas.R * r2 * T;
     }
-    s.PR4[c] = make_double4(pr[0], pr[1], pr[2], pr[3]);
+    st4(s.PR4 + c, make_double4(pr[0], pr[1], pr[2], pr[3]));
     if constexpr (MODEL == 2) s.PRx[c] = pr[4];
 }
 
@@ -1265,7 +1265,7 @@ __global__ void __launch_bounds__(BLOCK, MODEL == 2 ? 2 : 3) k_blocks(const Prm*
     loadU<MODEL>(s, nc, nb, Un);
     loadP<MODEL>(s, nc, nb, Pn);
     {
-        const double4 t = s.PR4[nb];
+        const double4 t = ld4(s.PR4 + nb);
         pr[0] = t.x; pr[1] = t.y; pr[2] = t.z; pr[3] = t.w;
         if constexpr (MODEL == 2) pr[4] = s.PRx[nb];
         // the last variable (nt, omega) is in no energy: e2Taprox returns the temperature itself
@@ -1398,7 +1398,7 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
         double* xnx = s.Xx[cur ^ 1];
         double xo[NV], xn[NV];
         {
-            double4 t = xo4[c];
+            double4 t = ld4(xo4 + c);
             xo[0] = t.x; xo[1] = t.y; xo[2] = t.z; xo[3] = t.w;
 #pragma unroll
             for (int k = 4; k < NV; k++) xo[k] = xox[(size_t)(k - 4) * nc + c];
@@ -1409,7 +1409,7 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
             gather_residual<MODEL>(p, m, s, c, Pc, R);
             storeR<MODEL>(s, nc, c, R);
         } else {
-            double4 t = s.R4[c];
+            double4 t = ld4(s.R4 + c);
             R[0] = t.x; R[1] = t.y; R[2] = t.z; R[3] = t.w;
 #pragma unroll
             for (int k = 4; k < NV; k++) R[k] = s.Rx[(size_t)(k - 4) * nc + c];
@@ -1445,7 +1445,7 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
                 if (j == 3 && ni <= 3) break;
                 const int nb = nbj[j];
                 double xb[NV];
-                double4 t = xo4[nb];
+                double4 t = ld4(xo4 + nb);
                 xb[0] = t.x; xb[1] = t.y; xb[2] = t.z; xb[3] = t.w;
 #pragma unroll
                 for (int k = 4; k < NV; k++) xb[k] = xox[(size_t)(k - 4) * nc + nb];
@@ -1460,7 +1460,7 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
             jacobi_update<MODEL>(s, nc, c, D, D4, R, y, xo, xn);
             dmax = fabs(xn[0] - xo[0]);
         }
-        xn4[c] = make_double4(xn[0], xn[1], xn[2], xn[3]);
+        st4(xn4 + c, make_double4(xn[0], xn[1], xn[2], xn[3]));
 #pragma unroll
         for (int k = 4; k < NV; k++) xnx[(size_t)(k - 4) * nc + c] = xn[k];
         if (LAST) {
@@ -1602,12 +1602,12 @@ __global__ void __launch_bounds__(LUSGS_THREADS) k_lusgs(const Prm* __restrict__
     const double D = s.dpart[c] + m.omega[c] / dt;
     double x[NV];
     if (FWD) {
-        double4 t4 = s.R4[c];
+        double4 t4 = ld4(s.R4 + c);
         x[0] = -t4.x; x[1] = -t4.y; x[2] = -t4.z; x[3] = -t4.w;
 #pragma unroll
         for (int k = 4; k < NV; k++) x[k] = -s.Rx[(size_t)(k - 4) * nc + c];
     } else {
-        double4 t4 = s.X4[0][c];
+        double4 t4 = ld4(s.X4[0] + c);
         x[0] = D * t4.x; x[1] = D * t4.y; x[2] = D * t4.z; x[3] = D * t4.w;
 #pragma unroll
         for (int k = 4; k < NV; k++) x[k] = D * s.Xx[0][(size_t)(k - 4) * nc + c];
@@ -1636,7 +1636,7 @@ __global__ void __launch_bounds__(LUSGS_THREADS) k_lusgs(const Prm* __restrict__
         double Pn[NP], dn[NV], dF[NV];
         loadP<MODEL>(s, nc, nb, Pn);
         {
-            double4 t4 = src4[nb];
+            double4 t4 = ld4(src4 + nb);
             dn[0] = t4.x; dn[1] = t4.y; dn[2] = t4.z; dn[3] = t4.w;
 #pragma unroll
             for (int k = 4; k < NV; k++) dn[k] = srcx[(size_t)(k - 4) * nc + nb];
@@ -1717,7 +1717,7 @@ __global__ void __launch_bounds__(BLOCK) k_update(const Prm* __restrict__ P, con
     const int nc = m.nc;
     double U[NV], W[NP];
     loadU<MODEL>(s, nc, c, U);
-    double4 t4 = s.X4[1][c];
+    double4 t4 = ld4(s.X4[1] + c);
     U[0] += t4.x; U[1] += t4.y; U[2] += t4.z; U[3] += t4.w;
 #pragma unroll
     for (int k = 4; k < NV; k++) U[k] += s.Xx[1][(size_t)(k - 4) * nc + c];
