@@ -1360,8 +1360,11 @@ __device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, dou
 // (209,825 quads, FP32) 38.7 -> 23.8 us, SST airfoil pack 22 % faster per pass. SA's register budget is 96 (640
 // threads per SM): at the compiler's own 64 the plate's sweep takes 28.6 us, at 80 23.0 but the SA pack 5 % more;
 // Euler and SST are fastest at the compiler's choice (Euler held to 48: 16.7 us, SST held to 96 or 128: 2-5 % slower).
-template <int MODEL, bool LAST, bool FIRST, int SB, bool F32>
-__global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+//
+// On small meshes a sweep is one chain of loads: EARLY issues the gathers before the halt and early-exit flags arrive,
+// for registers that cost more than the chain once several waves hide it (sweep_early: where the line lies).
+template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, bool EARLY = false>
+__global__ void __launch_bounds__(SB, MODEL == 1 && !EARLY ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
                                               const __grid_constant__ State s, int sweep, int cur, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
@@ -1387,18 +1390,25 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
         if (ni > 3) nbj[3] = m.fnb[3 * nc + c];
     }
     pdl_wait();
+    const double4* const xo4 = s.X4[cur];
+    const double* const xox = s.Xx[cur];
+    // EARLY: the increments are under way before the flags that may make them needless are known
+    double4 x4c = make_double4(0.0, 0.0, 0.0, 0.0), x4n[EARLY ? 3 : 1];
+    if (EARLY && valid) {
+        x4c = ld4(xo4 + c);
+#pragma unroll
+        for (int j = 0; j < (EARLY ? 3 : 1); j++) x4n[j] = ld4(xo4 + nbj[j]);
+    }
     if (halted(sc)) return;
     bool conv = !FIRST && sweep > 0 && bitsd(sc->sweep_max[sweep - 1]) < 1e-14;
     double dmax = 0.0;
     double R[NV];
     if (valid) {
-        const double4* xo4 = s.X4[cur];
-        const double* xox = s.Xx[cur];
         double4* xn4 = s.X4[cur ^ 1];
         double* xnx = s.Xx[cur ^ 1];
         double xo[NV], xn[NV];
         {
-            double4 t = ld4(xo4 + c);
+            double4 t = EARLY ? x4c : ld4(xo4 + c);
             xo[0] = t.x; xo[1] = t.y; xo[2] = t.z; xo[3] = t.w;
 #pragma unroll
             for (int k = 4; k < NV; k++) xo[k] = xox[(size_t)(k - 4) * nc + c];
@@ -1445,7 +1455,7 @@ __global__ void __launch_bounds__(SB, MODEL == 1 ? 640 / SB : 1) k_sweep(const P
                 if (j == 3 && ni <= 3) break;
                 const int nb = nbj[j];
                 double xb[NV];
-                double4 t = ld4(xo4 + nb);
+                double4 t = EARLY && j < 3 ? x4n[EARLY && j < 3 ? j : 0] : ld4(xo4 + nb);
                 xb[0] = t.x; xb[1] = t.y; xb[2] = t.z; xb[3] = t.w;
 #pragma unroll
                 for (int k = 4; k < NV; k++) xb[k] = xox[(size_t)(k - 4) * nc + nb];
