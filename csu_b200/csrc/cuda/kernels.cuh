@@ -272,8 +272,8 @@ constexpr int grad_blocks()
     return MODEL == 0 ? 6 : (MODEL == 1 ? 5 : 4);
 }
 
-template <int MODEL, bool DBG, int LSQ>
-__global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), grad_blocks<MODEL>())
+template <int MODEL, bool DBG, int LSQ, bool SMALL = false>
+__global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2 : grad_blocks<MODEL>())
     k_grad(const Prm* __restrict__ P, const __grid_constant__ Mesh m, const __grid_constant__ State s)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
