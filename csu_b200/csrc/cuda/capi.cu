@@ -1050,20 +1050,41 @@ static void launch_blocks(csu_ctx* x)
     else cudaEventRecord(x->ev_join, x->side);
 }
 
+using SweepKernel = void (*)(const Prm*, const Mesh, const State, int, int, int);
+
+// Whether the Euler and laminar sweeps trade registers for more blocks per SM: once the mesh is more than one wave of five
+// 128-cell blocks. Per iteration with 16 sweeps, compiler's registers -> 56: 160,000 cells FP64 216 -> 210 us, FP32 189 ->
+// 169, laminar FP32 262 -> 245; 80,000 cells, one wave, 118 -> 128, 106 -> 123, 146 -> 164.
+static bool sweep_wide(const csu_ctx* x)
+{
+    return x->model == 0 && x->L.nc > 5 * 128 * x->sm_count;
+}
+
+template <int MODEL, int SB, int MODE>
+static SweepKernel sweep_kernel_mode(const csu_ctx* x, bool first, bool last)
+{
+    if (x->cfg.implicit_fp32)
+        return first ? (last ? k_sweep<MODEL, true, true, SB, true, MODE> : k_sweep<MODEL, false, true, SB, true, MODE>)
+                     : (last ? k_sweep<MODEL, true, false, SB, true, MODE> : k_sweep<MODEL, false, false, SB, true, MODE>);
+    return first ? (last ? k_sweep<MODEL, true, true, SB, false, MODE> : k_sweep<MODEL, false, true, SB, false, MODE>)
+                 : (last ? k_sweep<MODEL, true, false, SB, false, MODE> : k_sweep<MODEL, false, false, SB, false, MODE>);
+}
+
+// the sweep in blocks of SB cells
+template <int MODEL, int SB>
+static SweepKernel sweep_kernel(const csu_ctx* x, bool first, bool last)
+{
+    if constexpr (MODEL == 0) {
+        if (sweep_wide(x)) return sweep_kernel_mode<MODEL, SB, SWEEP_WIDE>(x, first, last);
+    }
+    return sweep_kernel_mode<MODEL, SB, SWEEP_PLAIN>(x, first, last);
+}
+
 template <int MODEL, int SB>
 static void launch_sweep_sb(csu_ctx* x, int m, int n)
 {
-    if (m == 0) {
-        auto* k = x->cfg.implicit_fp32
-                      ? (m == n - 1 ? k_sweep<MODEL, true, true, SB, true> : k_sweep<MODEL, false, true, SB, true>)
-                      : (m == n - 1 ? k_sweep<MODEL, true, true, SB, false> : k_sweep<MODEL, false, true, SB, false>);
-        launch(x, k, x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
-    } else {
-        auto* k = x->cfg.implicit_fp32
-                      ? (m == n - 1 ? k_sweep<MODEL, true, false, SB, true> : k_sweep<MODEL, false, false, SB, true>)
-                      : (m == n - 1 ? k_sweep<MODEL, true, false, SB, false> : k_sweep<MODEL, false, false, SB, false>);
-        launch(x, k, x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
-    }
+    launch(x, sweep_kernel<MODEL, SB>(x, m == 0, m == n - 1), x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur,
+           x->max_ni);
 }
 
 // Whether the sweeps after the first gather before they know the flags (k_sweep's EARLY). Per iteration with 16 sweeps:
@@ -1081,8 +1102,8 @@ static void launch_sweep(csu_ctx* x, int m, int n)
     if (m > 0 && MODEL < 2 && sweep_early(x)) {
         constexpr int M = MODEL < 2 ? MODEL : 0, SB = 64;
         auto* k = x->cfg.implicit_fp32
-                      ? (m == n - 1 ? k_sweep<M, true, false, SB, true, true> : k_sweep<M, false, false, SB, true, true>)
-                      : (m == n - 1 ? k_sweep<M, true, false, SB, false, true> : k_sweep<M, false, false, SB, false, true>);
+                      ? (m == n - 1 ? k_sweep<M, true, false, SB, true, SWEEP_EARLY> : k_sweep<M, false, false, SB, true, SWEEP_EARLY>)
+                      : (m == n - 1 ? k_sweep<M, true, false, SB, false, SWEEP_EARLY> : k_sweep<M, false, false, SB, false, SWEEP_EARLY>);
         launch(x, k, x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
         x->launches++;
         tmark(x, KSWEEP);
@@ -1391,20 +1412,9 @@ static int time_sweep_shape(csu_ctx* x, int sb, int reps, cudaEvent_t e0, cudaEv
     CK(cudaMemcpy2DAsync(&x->st.sc[0].sweep_max[slot - 1], sizeof(Scalars), big.data(), sizeof(unsigned long long),
                          sizeof(unsigned long long), x->nsolve, cudaMemcpyHostToDevice, x->stream));
     auto launch = [&]() {
-        switch (sb) {
-        case 64:
-            (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 64, true> : k_sweep<MODEL, false, false, 64, false>)
-                <<<x->gb_c * (BLOCK / 64), 64, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
-            break;
-        case 256:
-            (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 256, true> : k_sweep<MODEL, false, false, 256, false>)
-                <<<x->gb_c, 256, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
-            break;
-        default:
-            (x->cfg.implicit_fp32 ? k_sweep<MODEL, false, false, 128, true> : k_sweep<MODEL, false, false, 128, false>)
-                <<<x->gb_c * 2, 128, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
-            break;
-        }
+        const SweepKernel k = sb == 64 ? sweep_kernel<MODEL, 64>(x, false, false)
+                              : sb == 256 ? sweep_kernel<MODEL, 256>(x, false, false) : sweep_kernel<MODEL, 128>(x, false, false);
+        k<<<x->gb_c * (BLOCK / sb), sb, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
     };
     launch();
     CK(cudaEventRecord(e0, x->stream));

@@ -1363,11 +1363,16 @@ __device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, dou
 //
 // On small meshes a sweep is one chain of loads: EARLY issues the gathers before the halt and early-exit flags arrive,
 // for registers that cost more than the chain once several waves hide it (sweep_early: where the line lies).
-template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, bool EARLY = false>
-__global__ void __launch_bounds__(SB, MODEL == 1 && !EARLY ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
+//
+// On meshes of more than one wave of the compiler's 88 registers WIDE holds Euler and laminar to 56 (sweep_wide).
+enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
+
+template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, int MODE = SWEEP_PLAIN>
+__global__ void __launch_bounds__(SB, MODE == SWEEP_WIDE ? 1152 / SB : MODEL == 1 && MODE == SWEEP_PLAIN ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
                                               const __grid_constant__ State s, int sweep, int cur, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
+    constexpr bool EARLY = MODE == SWEEP_EARLY;
     static_assert(BLOCK % SB == 0, "sweep blocks tile the cell blocks");
     // SB-thread blocks: BLOCK / SB of them cover one cell block of the solve map
     const int sid = s.bsolve ? s.bsolve[blockIdx.x / (BLOCK / SB)] : 0;
