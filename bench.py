@@ -131,22 +131,23 @@ def alg_bytes(case):
     W = 40                      # r u v p + T
     G = 96                      # gradient x, y and limiter of r u v p
     return {
-        # W, npts, omega, x87 LSQ constants (a b c det + reciprocal), nei + dx dy + edge vectors per slot,
+        # W, npts, omega factor, least-squares constants over the determinant, nei + dx dy + edge vectors per slot,
         # ghost geometry per boundary face, gradients/limiter out
-        "grad": nc * (W + 4 + 8 + 56 + G) + slots * (4 + 16 + 16) + nb * 28,
+        "grad": nc * (W + 4 + 8 + 48 + G) + slots * (4 + 16 + 16) + nb * 28,
         # face index/normal/|dS|/two centre offsets + flux out; boundary face data + flux out; cell W and G in
         "flux": nf * (8 + 16 + 8 + 32 + 32) + nb * (4 + 4 + 16 + 8 + 32) + nc * (W + G),
-        # DPLUR diagonal (k_impl without R): W, counts, omega; per slot fslot; face cells, normal, |dS|;
+        # DPLUR diagonal (k_impl without R): W, counts, omega; per slot fslot; per face its two spectral radii;
         # boundary normal, |dS|; Omega/Lc and diagonal out
-        "impl": nc * (W + 8 + 8 + 8 + 8) + slots * 4 + nf * 32 + nb * 24,
-        # U and W of every cell (as a neighbour), counts; face cells, normal, |dS|; per interior slot fslot +
-        # the 16 FP64 block out
-        "blocks": nc * (32 + W + 4) + nf * 32 + nint * (4 + 128),
-        # mean of the four sweeps of an iteration: x in, x out, counts, R, diagonal part, omega; per interior
-        # slot its neighbour + 16 FP64 block; the first sweep also reads W, the face fluxes and the slots
-        # (R gather), the last reads and writes U and writes W
-        "sweep": nc * (32 + 32 + 4 + 32 + 8 + 8) + nint * (4 + 128)
-                 + (nc * W + (nf + nb) * 32 + slots * 4 + nc * (32 + 32 + W)) // 4,
+        "impl": nc * (W + 8 + 8 + 8 + 8) + slots * 4 + nf * 16 + nb * 24,
+        # k_side: U, W in, stepped pressures out; face cells, normal, |dS| in, spectral radii out. k_blocks: U, W and
+        # those pressures of every cell (as a neighbour), counts; face normal, |dS|; per interior slot fslot,
+        # neighbour and the 15 FP64 entries that are not zero out
+        "blocks": nc * (32 + W + 32) + nf * (8 + 24 + 16) + nc * (32 + W + 32 + 4) + nf * 24 + nint * (8 + 120),
+        # mean of the four sweeps of an iteration: x in, x out, counts, R, diagonal; per interior slot its neighbour +
+        # the block's 15 entries; the first sweep also reads W, the face fluxes, the slots (R gather) and the diagonal's
+        # parts, the last reads and writes U and writes W
+        "sweep": nc * (32 + 32 + 4 + 32 + 8) + nint * (4 + 120)
+                 + (nc * W + (nf + nb) * 32 + slots * 4 + nc * 16 + nc * (32 + 32 + W)) // 4,
     }
 
 

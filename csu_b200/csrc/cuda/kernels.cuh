@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(BLOCK) k_prim(const Prm* __restrict__ P, const
 // lanes share a cell's double4 records), the certified solve keeps every x87 rounding in its bound instead of in
 // the arithmetic (lsq_decide), the two branches of the limiter are one, and the 1-3 % of components left undecided
 // are finished together, one per thread of the block. Against one thread per cell with the x87 sums emulated in
-// every component and k_grad_fix behind it: 3,049 mixed cells 36.7 -> 16.7 us, 30,000 laminar 37.9 -> 22, 160,000
-// triangles 68 -> 59, 500,000 170 -> 147, the 209,825-quad SA plate 109 -> 100 (events, launch gap included; at
+// every component, the rare ones in a kernel behind it: 3,049 mixed cells 36.7 -> 16.7 us, 30,000
+// laminar 37.9 -> 22, 160,000 triangles 68 -> 59, 500,000 170 -> 147, the 209,825-quad SA plate 109 -> 100 (events, launch gap included; at
 // 160,000 triangles 8 % of the measured copy bandwidth for the 50 MB it must move). Measured and dropped: the
 // undecided components where they arise (67 us; a warp has one nearly every time), in a kernel of their own
 // (137 us at 500,000, but 28 us at 3,049), on a warp of their own beside the next group's (109 us).
