@@ -176,7 +176,6 @@ __device__ __noinline__ double lsq_slot_x87(const Prm& p, const Mesh& m, const S
     const X80 det = x80_add(x80_mul(K[0], K[2]), x80_neg(x80_mul(K[1], K[1])));
     // (c A - b B) / det, (-b A + a B) / det: A + B and B + A round alike
     const X80 N = x80_add(x80_mul(y ? K[0] : K[2], X), x80_mul(x80_neg(K[1]), Y));
-    atomicAdd(s.lsq_x87, 1ULL);
     return x80_to_double(x80_div(N, det));
 }
 
@@ -413,17 +412,21 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2
             const double2 qb = m.lq[nc + c2], qr = m.lq[3 * nc + c2];
             const DD kb = {qb.x, qb.y}, R = {qr.x, qr.y};
             double gx = sdu[q][6][l], gy = sdu[q][7][l];
+            bool left = false; // either component left to the integer model: the variable counts once
 #pragma unroll 1
             for (unsigned nd = w >> 8; nd; nd &= nd - 1) {
                 const bool y = (nd & 1u) == 0;
                 const double2 qk = m.lq[(y ? 0 : 2) * nc + c2];
                 const DD k1 = {qk.x, qk.y};
                 double g = 0.0;
-                if (!ok || !lsq_exact_numerator(k1, kb, R, y ? Y : X, y ? X : Y, &g))
+                if (!ok || !lsq_exact_numerator(k1, kb, R, y ? Y : X, y ? X : Y, &g)) {
                     g = lsq_slot_x87<MODEL>(p, m, s, c2, q < NV ? slot2p(q) : 4, y);
+                    left = true;
+                }
                 if (y) gy = g;
                 else gx = g;
             }
+            if (left) atomicAdd(s.lsq_x87, 1ULL);
             grad_finish<MODEL>(p, m, s, sc, c2, q, np, gx, gy, sdu[q][4][l], sdu[q][5][l]);
         }
     }
