@@ -125,58 +125,48 @@ __device__ __forceinline__ double limiter_eps2(const Prm& p, const Scalars* sc, 
     return a2 * a2;
 }
 
-// primitive vi (T: 4) of cell c
-__device__ __forceinline__ double cell_value(const State& s, int nc, int c, int vi)
+// The integer x87 model's constants of cell c: a, b, c (exact as double-doubles), det = a c - b b as the host's long
+// double rounds it (solver.c:1063-1073), and the reciprocal of its significand.
+struct LsqX87 {
+    X80 a, b, c, det;
+    unsigned long long rv;
+};
+
+__device__ __forceinline__ LsqX87 lsq_x87_consts(const Mesh& m, int c)
 {
-    return vi < 4 ? reinterpret_cast<const double*>(s.W4 + c)[vi] : vi == 4 ? s.WT[c] : s.Wx[(size_t)(vi - 5) * nc + c];
+    const double2 qa = m.lq[c], qb = m.lq[m.nc + c], qc = m.lq[2 * m.nc + c];
+    LsqX87 K;
+    K.a = x80_add(x80_from_double(qa.x), x80_from_double(qa.y));
+    K.b = x80_add(x80_from_double(qb.x), x80_from_double(qb.y));
+    K.c = x80_add(x80_from_double(qc.x), x80_from_double(qc.y));
+    K.det = x80_add(x80_mul(K.a, K.c), x80_neg(x80_mul(K.b, K.b)));
+    K.rv = K.det.m ? x80_recip(K.det.m) : 0;
+    return K;
 }
 
-// primitive vi (T: 4) of the neighbour (cell or ghost) in slot j of cell c
-template <int MODEL>
-__device__ __forceinline__ double nei_value(const Prm& p, const Mesh& m, const State& s, int c, int j, int vi)
+// Both gradient components of cell c from the differences du(j) of a variable to its neighbours, every operation with
+// the integer x87 model: the rare variables nothing else can decide, and every variable with CSU_LSQ=x87. Bound by
+// integer issue: the components share the sums, a cell's variables (k_grad with LSQ 1) the constants.
+template <typename DU>
+__device__ __forceinline__ double2 lsq_x87(const Mesh& m, const LsqX87& K, int c, int np, DU du)
 {
-    constexpr int NP = Model<MODEL>::NP;
-    const int nc = m.nc, n = m.nei[j * nc + c];
-    if (n < nc) return cell_value(s, nc, n, vi);
-    const int b = n - nc;
-    double P0[NP], Pn[NP];
-    loadP<MODEL>(s, nc, c, P0);
-    const double2 dSv = m.bn[b];
-    ghost_state<MODEL>(p, m.bflag[b], dSv.x, dSv.y, m.bds[b], P0, m.wall_d ? m.wall_d[c] : 0.0, Pn);
-    double v = Pn[0];
-#pragma unroll
-    for (int k = 1; k < NP; k++)
-        if (k == vi) v = Pn[k];
-    return v;
-}
-
-// Gradient component (x, or y) of cell c for primitive vi with the integer x87 model, gathering the neighbours
-// again: the rare components nothing else can decide, and every component with CSU_LSQ=x87.
-template <int MODEL>
-__device__ __noinline__ double lsq_slot_x87(const Prm& p, const Mesh& m, const State& s, int c, int vi, bool y)
-{
-    const int nc = m.nc;
-    const double u0 = cell_value(s, nc, c, vi);
-    X80 X = x80_zero(0), Y = x80_zero(0);
-    const int np = m.npts[c];
+    X80 A = x80_zero(0), B = x80_zero(0);
 #pragma unroll 1
     for (int j = 0; j < np; j++) {
-        const double du = nei_value<MODEL>(p, m, s, c, j, vi) - u0;
-        const double2 d = m.ld[j * nc + c];
-        X = x80_add(X, x80_from_double((y ? d.y : d.x) * du));
-        Y = x80_add(Y, x80_from_double((y ? d.x : d.y) * du));
+        const double2 d = m.ld[j * m.nc + c];
+        const double v = du(j);
+        A = x80_add(A, x80_from_double(d.x * v));
+        B = x80_add(B, x80_from_double(d.y * v));
     }
-    // a, b, c (exact as double-doubles) and det = a c - b b, rounded as the host's long double (solver.c:1063-1073)
-    X80 K[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        const double2 v = m.lq[q * nc + c];
-        K[q] = x80_add(x80_from_double(v.x), x80_from_double(v.y));
-    }
-    const X80 det = x80_add(x80_mul(K[0], K[2]), x80_neg(x80_mul(K[1], K[1])));
-    // (c A - b B) / det, (-b A + a B) / det: A + B and B + A round alike
-    const X80 N = x80_add(x80_mul(y ? K[0] : K[2], X), x80_mul(x80_neg(K[1]), Y));
-    return x80_to_double(x80_div(N, det));
+    const X80 nx = x80_add(x80_mul(K.c, A), x80_neg(x80_mul(K.b, B)));
+    const X80 ny = x80_add(x80_mul(x80_neg(K.b), A), x80_mul(K.a, B));
+    return make_double2(x80_to_double(x80_div_pre(nx, K.det, K.rv)), x80_to_double(x80_div_pre(ny, K.det, K.rv)));
+}
+
+// the same from differences in shared memory, out of line: k_grad's undecided variables
+static __device__ __noinline__ double2 lsq_x87_left(const Mesh& m, int c, int np, const double* du)
+{
+    return lsq_x87(m, lsq_x87_consts(m, c), c, np, [=](int j) { return du[j * GRAD_CELLS]; });
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -265,14 +255,17 @@ __device__ __forceinline__ void grad_finish(const Prm& p, const Mesh& m, const S
 
 // Blocks per SM of k_grad's register budget (64 registers; SST 72): with fewer the loads' latency shows (160,000
 // triangles, Euler: 4 blocks 68 us, 5 61, 6 59), with more the undecided components' code spills into the rest (8: 71).
-template <int MODEL>
+// SMALL: small meshes' undecided components without spills. LSQ 1: 80 registers (200,000 cells, RK5 with CSU_LSQ=x87:
+// 922 us an iteration; two blocks of 96 registers 1,025).
+template <int MODEL, int LSQ, bool SMALL>
 constexpr int grad_blocks()
 {
-    return MODEL == 0 ? 6 : (MODEL == 1 ? 5 : 4);
+    if (LSQ == 1) return 800 / (GRAD_CELLS * (Model<MODEL>::NV + 1));
+    return SMALL ? 2 : MODEL == 0 ? 6 : (MODEL == 1 ? 5 : 4);
 }
 
 template <int MODEL, bool DBG, int LSQ, bool SMALL = false>
-__global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2 : grad_blocks<MODEL>())
+__global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), grad_blocks<MODEL, LSQ, SMALL>())
     k_grad(const Prm* __restrict__ P, const __grid_constant__ Mesh m, const __grid_constant__ State s)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
@@ -281,6 +274,7 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2
     __shared__ double sdu[LSQ == 2 ? NV + 1 : 1][8][GRAD_CELLS];
     __shared__ unsigned short list[LSQ == 2 ? (NV + 1) * GRAD_CELLS : 1];
     __shared__ unsigned nlist;
+    __shared__ LsqX87 sk[LSQ == 1 ? GRAD_CELLS : 1];
     const int sid = s.bsolve ? s.bsolve[blockIdx.x / (BLOCK / GRAD_CELLS)] : 0;
     const Prm& p = P[sid];
     const Scalars* const sc = s.sc + sid;
@@ -306,6 +300,12 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2
             nj[j] = m.nei[j * nc + cr];
             d[j] = (LSQ == 0 ? m.lw : m.ld)[j * nc + cr];
         }
+    }
+    if (LSQ == 1) {
+        // padding rows hold zeros, whose constants nothing reads
+        if (threadIdx.x < GRAD_CELLS)
+            sk[threadIdx.x] = lsq_x87_consts(m, min(blockIdx.x * GRAD_CELLS + threadIdx.x, nc - 1));
+        __syncthreads();
     }
     pdl_wait();
     const bool stop = halted_behind(p, sc);
@@ -360,8 +360,11 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2
                 }
             }
         } else if (LSQ == 1) {
-            gx = lsq_slot_x87<MODEL>(p, m, s, c, vi, false);
-            gy = lsq_slot_x87<MODEL>(p, m, s, c, vi, true);
+            const double2 g = lsq_x87(m, sk[lane], c, np, [&](int j) {
+                return j == 0 ? du[0] : j == 1 ? du[1] : j == 2 ? du[2] : du[3];
+            });
+            gx = g.x;
+            gy = g.y;
         } else {
             // solverCalcGrad3 (solver.c:1063-1073): double products summed in long double, then
             // dUx = (c A - b B) / (a c - b b), dUy = (-b A + a B) / (a c - b b) in long double
@@ -420,7 +423,8 @@ __global__ void __launch_bounds__(GRAD_CELLS * (Model<MODEL>::NV + 1), SMALL ? 2
                 const DD k1 = {qk.x, qk.y};
                 double g = 0.0;
                 if (!ok || !lsq_exact_numerator(k1, kb, R, y ? Y : X, y ? X : Y, &g)) {
-                    g = lsq_slot_x87<MODEL>(p, m, s, c2, q < NV ? slot2p(q) : 4, y);
+                    const double2 g2 = lsq_x87_left(m, c2, np, &sdu[q][0][l]);
+                    g = y ? g2.y : g2.x;
                     left = true;
                 }
                 if (y) gy = g;
