@@ -12,6 +12,7 @@
 #include <tuple>
 #include "csu_gpu.h"
 #include "kernels.cuh"
+#include "launch_rules.h"
 
 extern "C" {
 #include "../host/layout.h"
@@ -1052,14 +1053,6 @@ static void launch_blocks(csu_ctx* x)
 
 using SweepKernel = void (*)(const Prm*, const Mesh, const State, int, int, int);
 
-// Whether the Euler and laminar sweeps trade registers for more blocks per SM: once the mesh is more than one wave of five
-// 128-cell blocks. Per iteration with 16 sweeps, compiler's registers -> 56: 160,000 cells FP64 216 -> 210 us, FP32 189 ->
-// 169, laminar FP32 262 -> 245; 80,000 cells, one wave, 118 -> 128, 106 -> 123, 146 -> 164.
-static bool sweep_wide(const csu_ctx* x)
-{
-    return x->model == 0 && x->L.nc > 5 * 128 * x->sm_count;
-}
-
 template <int MODEL, int SB, int MODE>
 static SweepKernel sweep_kernel_mode(const csu_ctx* x, bool first, bool last)
 {
@@ -1075,7 +1068,7 @@ template <int MODEL, int SB>
 static SweepKernel sweep_kernel(const csu_ctx* x, bool first, bool last)
 {
     if constexpr (MODEL == 0) {
-        if (sweep_wide(x)) return sweep_kernel_mode<MODEL, SB, SWEEP_WIDE>(x, first, last);
+        if (sweep_wide(MODEL, x->cfg.implicit_fp32, x->L.nc, x->sm_count)) return sweep_kernel_mode<MODEL, SB, SWEEP_WIDE>(x, first, last);
     }
     return sweep_kernel_mode<MODEL, SB, SWEEP_PLAIN>(x, first, last);
 }

@@ -1371,7 +1371,8 @@ __device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, dou
 // On small meshes a sweep is one chain of loads: EARLY issues the gathers before the halt and early-exit flags arrive,
 // for registers that cost more than the chain once several waves hide it (sweep_early: where the line lies).
 //
-// On meshes of more than one wave of the compiler's 88 registers WIDE holds Euler and laminar to 56 (sweep_wide).
+// WIDE holds Euler and laminar, 88 registers by themselves, to 56 in blocks of 64 and 128 cells and to 64 in blocks of
+// 256 (sweep_wide: on which meshes).
 enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
 
 template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, int MODE = SWEEP_PLAIN>

@@ -1,0 +1,27 @@
+// launch_rules.h -- which build of the DPLUR sweep a mesh gets, as functions of the mesh and the device alone.
+#pragma once
+
+namespace csu {
+
+// waves of `cells` cells on `sms` multiprocessors that hold `per_sm` of them at a time
+constexpr long long sweep_waves(long long cells, int per_sm, int sms)
+{
+    return (cells + (long long)per_sm * sms - 1) / ((long long)per_sm * sms);
+}
+
+// Whether the Euler and laminar sweeps trade registers for more cells in flight (k_sweep's WIDE): 1,152 per
+// multiprocessor instead of 640 at the compiler's own count. The build with fewer registers is slower cell by cell (its
+// loads are less far ahead), so it has to save waves: half of them with FP64 blocks, a third with FP32 blocks. Per
+// iteration with 16 sweeps on 148 multiprocessors, PLAIN -> WIDE, wide / plain waves in brackets:
+//   laminar FP32  160,904 cells 310 -> 279 us (1/2), 185,606 341 -> 388 (2/2), 210,136 426 -> 412 (2/3),
+//                 295,241 576 -> 521 (2/4), 350,514 818 -> 872 (3/4), 499,477 1,166 -> 1,114 (3/6)
+//   Euler FP64    168,100 245 -> 231 (1/2), 186,192 267 -> 324 (2/2), 210,222 339 -> 354 (2/3), 294,848 621 -> 607 (2/4),
+//                 380,072 767 -> 832 (3/5), 499,848 1,006 -> 1,005 (3/6), 599,850 1,176 -> 1,232 (4/7)
+constexpr bool sweep_wide(int model, bool fp32, long long cells, int sms)
+{
+    if (model != 0) return false;
+    const long long plain = sweep_waves(cells, 640, sms), wide = sweep_waves(cells, 1152, sms);
+    return fp32 ? 3 * wide <= 2 * plain : 2 * wide <= plain;
+}
+
+} // namespace csu

@@ -1,0 +1,35 @@
+"""The choice of sweep build (csu_b200/csrc/cuda/launch_rules.h), compiled for the host: WIDE only where it saves enough
+waves, the same choice for the same cells per multiprocessor, PLAIN for every mesh of one wave."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("rules") / "launch_rules_check")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-o", exe,
+                    os.path.join(ROOT, "tests", "native", "launch_rules_check.cpp")], check=True)
+
+    def ask(rows):
+        r = subprocess.run([exe], input="\n".join("%d %d %d %d" % q for q in rows), capture_output=True, text=True,
+                           check=True)
+        return [tuple(int(v) for v in line.split()) for line in r.stdout.splitlines()]
+    return ask
+
+
+# (cells per multiprocessor, FP64 WIDE, FP32 WIDE): either side of each line between wave counts
+LINES = [(640, 0, 0), (641, 1, 1), (1152, 1, 1), (1153, 0, 0), (1280, 0, 0), (1281, 0, 1), (1920, 0, 1), (1921, 1, 1),
+         (2304, 1, 1), (2305, 0, 0), (2560, 0, 0), (2561, 0, 1), (3200, 0, 1), (3201, 1, 1), (3456, 1, 1),
+         (3457, 0, 1)]
+
+
+@pytest.mark.parametrize("sms", [148, 132, 20])
+def test_wide_where_it_saves_waves(rules, sms):
+    for per_sm, f64, f32 in LINES:
+        got = rules([(0, 0, per_sm * sms, sms), (0, 1, per_sm * sms, sms), (1, 1, per_sm * sms, sms),
+                     (2, 0, per_sm * sms, sms)])
+        assert [g[0] for g in got] == [f64, f32, 0, 0], per_sm
