@@ -12,7 +12,6 @@
 #include <tuple>
 #include "csu_gpu.h"
 #include "kernels.cuh"
-#include "launch_rules.h"
 
 extern "C" {
 #include "../host/layout.h"
@@ -1363,7 +1362,7 @@ static int build_graph(csu_ctx* x, int gi)
 // iteration computes again before reading them; the timed sweep is a middle sweep that writes the spare
 // increment buffer (the next iteration's first sweep overwrites it) and uses the last early-exit slot pair,
 // cleared afterwards. Choices are cached per device, model, order, viscosity, block precision and size class
-// (half octaves of the cell count), so packs of a size class seen before take the cached shapes.
+// (tune_class), so packs of a size class seen before take the cached shapes.
 namespace {
 struct TuneKey {
     int dev, model, order, visc, blk32, implicit, size_class;
@@ -1471,7 +1470,7 @@ static int autotune(csu_ctx* x, bool force)
     if (env && strcmp(env, "0") == 0) return CSU_OK;
     if (x->L.nc < 16384 && !force) return CSU_OK;
     TuneKey key{x->device, x->model, x->cfg.order, x->prm.visc, x->cfg.implicit_fp32,
-                x->cfg.time_scheme, (int)floor(2.0 * log2((double)x->L.nc))};
+                x->cfg.time_scheme, tune_class(x->model, x->cfg.implicit_fp32, x->L.nc, x->sm_count)};
     int fb = x->flux_fb, sb = x->sweep_sb;
     bool hit = false;
     if (!force) {

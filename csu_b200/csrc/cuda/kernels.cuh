@@ -16,6 +16,7 @@
 // iteration sequences can be captured in one CUDA graph.
 #pragma once
 #include "engine.cuh"
+#include "launch_rules.h"
 
 namespace csu {
 
@@ -1373,8 +1374,6 @@ __device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, dou
 //
 // WIDE holds Euler and laminar, 88 registers by themselves, to 56 in blocks of 64 and 128 cells and to 64 in blocks of
 // 256 (sweep_wide: on which meshes).
-enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
-
 template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, int MODE = SWEEP_PLAIN>
 __global__ void __launch_bounds__(SB, MODE == SWEEP_WIDE ? 1152 / SB : MODEL == 1 && MODE == SWEEP_PLAIN ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
                                               const __grid_constant__ State s, int sweep, int cur, int slots)

@@ -1,5 +1,6 @@
 // launch_rules.h -- which build of the DPLUR sweep a mesh gets, as functions of the mesh and the device alone.
 #pragma once
+#include <math.h>
 
 namespace csu {
 
@@ -22,6 +23,18 @@ constexpr bool sweep_wide(int model, bool fp32, long long cells, int sms)
     if (model != 0) return false;
     const long long plain = sweep_waves(cells, 640, sms), wide = sweep_waves(cells, 1152, sms);
     return fp32 ? 3 * wide <= 2 * plain : 2 * wide <= plain;
+}
+
+// The builds of k_sweep.
+enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
+
+// Meshes that share the autotuner's choice: half octaves of the cell count, apart where the sweep build differs (a shape
+// timed on one build is wrong for the other: 360,000 cells Euler FP32 752 us an iteration with the shape of 300,000's
+// WIDE sweeps, 670 with its own).
+inline int tune_class(int model, bool fp32, long long cells, int sms)
+{
+    const int build = sweep_wide(model, fp32, cells, sms) ? SWEEP_WIDE : SWEEP_PLAIN;
+    return (int)floor(2.0 * log2((double)cells)) * 4 + build;
 }
 
 } // namespace csu

@@ -33,3 +33,13 @@ def test_wide_where_it_saves_waves(rules, sms):
         got = rules([(0, 0, per_sm * sms, sms), (0, 1, per_sm * sms, sms), (1, 1, per_sm * sms, sms),
                      (2, 0, per_sm * sms, sms)])
         assert [g[0] for g in got] == [f64, f32, 0, 0], per_sm
+
+
+def test_tune_class_separates_builds(rules):
+    """Meshes of one class have one sweep build, at every size from the smallest tuned mesh up."""
+    for fp32 in (0, 1):
+        seen = {}
+        for cells, (wide, cls) in zip(range(16384, 700000, 97), rules([(0, fp32, c, 148)
+                                                                       for c in range(16384, 700000, 97)])):
+            assert seen.setdefault(cls, wide) == wide, cells
+        assert set(seen.values()) == {0, 1}
