@@ -1079,19 +1079,10 @@ static void launch_sweep_sb(csu_ctx* x, int m, int n)
            x->max_ni);
 }
 
-// Whether the sweeps after the first gather before they know the flags (k_sweep's EARLY). Per iteration with 16 sweeps:
-// Euler FP64 5,000 cells 79 -> 69 us, 20,000 81 -> 74, 40,000 87 -> 94; Euler and laminar FP32 40,000 89 -> 83 and 108
-// -> 102, 80,000 106 -> 112 and 147 -> 155; SA FP64 20,000 125 -> 115, its FP32 and SST within 2 % either way.
-static bool sweep_early(const csu_ctx* x)
-{
-    if (x->model == 2) return false;
-    return x->L.nc <= (x->model == 0 && x->cfg.implicit_fp32 ? 45000 : 25000);
-}
-
 template <int MODEL>
 static void launch_sweep(csu_ctx* x, int m, int n)
 {
-    if (m > 0 && MODEL < 2 && sweep_early(x)) {
+    if (m > 0 && sweep_early(MODEL, x->cfg.implicit_fp32, x->L.nc, x->sm_count)) {
         constexpr int M = MODEL < 2 ? MODEL : 0, SB = 64;
         auto* k = x->cfg.implicit_fp32
                       ? (m == n - 1 ? k_sweep<M, true, false, SB, true, SWEEP_EARLY> : k_sweep<M, false, false, SB, true, SWEEP_EARLY>)

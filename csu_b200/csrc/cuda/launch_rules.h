@@ -25,6 +25,18 @@ constexpr bool sweep_wide(int model, bool fp32, long long cells, int sms)
     return fp32 ? 3 * wide <= 2 * plain : 2 * wide <= plain;
 }
 
+// Whether the sweeps after the first gather before they know the flags (k_sweep's EARLY): a shorter chain of loads for
+// more registers, which pays while few cells share a multiprocessor. The lines lie between the last size that gained and
+// the first that did not, per iteration with 16 sweeps on 148 multiprocessors (cells: PLAIN -> EARLY):
+//   Euler FP64    34,810 94.3 -> 90.3 us, 39,728 98.8 -> 101.9     laminar FP64  34,810 106.7 -> 102.0, 39,728 117.4 -> 119.9
+//   Euler FP32    44,987 99.9 -> 94.5, 49,611 106.7 -> 105.5, 55,402 108.5 -> 108.9
+//   laminar FP32  44,987 114.5 -> 108.8, 49,611 122.9 -> 122.4, 55,402 128.6 -> 129.2
+//   SA FP64       25,264 124.1 -> 115.2, 30,193 130.4 -> 130.4     SA FP32       25,264 114.2 -> 113.5, 34,810 120.5 -> 121.2
+constexpr bool sweep_early(int model, bool fp32, long long cells, int sms)
+{
+    return model < 2 && cells <= (long long)sms * (model == 1 ? 192 : fp32 ? 320 : 256);
+}
+
 // The builds of k_sweep.
 enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
 
@@ -33,7 +45,9 @@ enum { SWEEP_PLAIN, SWEEP_EARLY, SWEEP_WIDE };
 // WIDE sweeps, 670 with its own).
 inline int tune_class(int model, bool fp32, long long cells, int sms)
 {
-    const int build = sweep_wide(model, fp32, cells, sms) ? SWEEP_WIDE : SWEEP_PLAIN;
+    const int build = sweep_early(model, fp32, cells, sms)  ? SWEEP_EARLY
+                      : sweep_wide(model, fp32, cells, sms) ? SWEEP_WIDE
+                                                            : SWEEP_PLAIN;
     return (int)floor(2.0 * log2((double)cells)) * 4 + build;
 }
 

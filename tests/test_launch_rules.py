@@ -39,7 +39,16 @@ def test_tune_class_separates_builds(rules):
     """Meshes of one class have one sweep build, at every size from the smallest tuned mesh up."""
     for fp32 in (0, 1):
         seen = {}
-        for cells, (wide, cls) in zip(range(16384, 700000, 97), rules([(0, fp32, c, 148)
-                                                                       for c in range(16384, 700000, 97)])):
-            assert seen.setdefault(cls, wide) == wide, cells
-        assert set(seen.values()) == {0, 1}
+        sizes = range(16384, 700000, 97)
+        for cells, (wide, cls, early) in zip(sizes, rules([(0, fp32, c, 148) for c in sizes])):
+            assert seen.setdefault(cls, (wide, early)) == (wide, early), cells
+        assert set(seen.values()) == {(0, 0), (0, 1), (1, 0)}
+
+
+@pytest.mark.parametrize("sms", [148, 132, 20])
+def test_early_by_cells_per_multiprocessor(rules, sms):
+    """The line of EARLY scales with the device, as WIDE's does."""
+    for model, fp32, per_sm in ((0, 0, 256), (0, 1, 320), (1, 0, 192), (1, 1, 192), (2, 0, 0), (2, 1, 0)):
+        at, above = rules([(model, fp32, per_sm * sms, sms), (model, fp32, per_sm * sms + 1, sms)])
+        assert (at[2], above[2]) == (int(per_sm > 0), 0)
+        assert not (at[0] or above[0])
