@@ -150,7 +150,7 @@ struct csu_ctx {
     int fin_bsel = 0;
     int max_ni = 4;          // most interior faces of a cell (k_blocks covers slots [0, max_ni))
     int flux_fb = 64;        // faces per k_flux block (one of FLUX_BLOCKS)
-    int sweep_sb = 128;      // cells per DPLUR sweep block (one of SWEEP_BLOCKS)
+    int sweep_sb = 128;      // cells per DPLUR sweep block (one of SWEEP_BLOCKS; EARLY sweeps: 64)
     bool tuned = false;      // launch shapes chosen (csu_autotune, or its cache on the first iteration)
     int device = 0;          // the CUDA device current when the context was made (its memory lives there)
     int sm_count = 148;      // that device's multiprocessors
@@ -627,6 +627,12 @@ static int launch_lim3(csu_ctx* x)
     return CSU_OK;
 }
 
+// Whether the context's DPLUR sweeps are the EARLY build, whose blocks have 64 cells
+static bool early_sweeps(const csu_ctx* x)
+{
+    return x->cfg.time_scheme == CSU_TS_DPLUR && sweep_early(x->model, x->cfg.implicit_fp32, x->L.nc, x->sm_count);
+}
+
 static int ctx_setup(csu_ctx* x)
 {
     int st;
@@ -663,6 +669,7 @@ static int ctx_setup(csu_ctx* x)
     if (e != cudaSuccess) return cuda_fail(e, "context setup");
     x->gb_c = (x->L.nc + BLOCK - 1) / BLOCK;
     if (x->L.nint) x->max_ni = max_nint(x->L); // packs set it from their solves
+    if (early_sweeps(x)) x->sweep_sb = 64;
     plan_l2_window(x);
     if (!x->is_pack && (st = upload_mesh(x))) return st; // packs: pack_build fills the mesh rows
     x->prm = x->prms[0];
@@ -1082,7 +1089,7 @@ static void launch_sweep_sb(csu_ctx* x, int m, int n)
 template <int MODEL>
 static void launch_sweep(csu_ctx* x, int m, int n)
 {
-    if (m > 0 && sweep_early(MODEL, x->cfg.implicit_fp32, x->L.nc, x->sm_count)) {
+    if (m > 0 && early_sweeps(x)) {
         constexpr int M = MODEL < 2 ? MODEL : 0, SB = 64;
         auto* k = x->cfg.implicit_fp32
                       ? (m == n - 1 ? k_sweep<M, true, false, SB, true, SWEEP_EARLY> : k_sweep<M, false, false, SB, true, SWEEP_EARLY>)
@@ -1434,7 +1441,8 @@ static int tune_shapes(csu_ctx* x, int* fb_out, int* sb_out)
         }
     }
     *sb_out = x->sweep_sb;
-    if (!st && x->cfg.time_scheme == CSU_TS_DPLUR) {
+    // EARLY sweeps have one shape
+    if (!st && x->cfg.time_scheme == CSU_TS_DPLUR && !early_sweeps(x)) {
         best = 1e30f;
         for (int sb : SWEEP_BLOCKS) {
             float ms = 0;
