@@ -1379,11 +1379,15 @@ static int time_flux_shape(csu_ctx* x, int fb, int reps, cudaEvent_t e0, cudaEve
 {
     const int save = x->flux_fb;
     x->flux_fb = fb;
-    x->chained = false;
     const long long l0 = x->launches;
+    // as the iteration launches it: DPLUR's flux starts when the kernel before it has ended, the others' overlap its tail
+    x->chained = false;
     launch_flux<MODEL>(x, 1);
     CK(cudaEventRecord(e0, x->stream));
-    for (int r = 0; r < reps; r++) launch_flux<MODEL>(x, 1);
+    for (int r = 0; r < reps; r++) {
+        if (x->cfg.time_scheme == CSU_TS_DPLUR) x->chained = false;
+        launch_flux<MODEL>(x, 1);
+    }
     CK(cudaEventRecord(e1, x->stream));
     x->flux_fb = save;
     x->launches = l0;
@@ -1401,14 +1405,15 @@ static int time_sweep_shape(csu_ctx* x, int sb, int reps, cudaEvent_t e0, cudaEv
     std::vector<unsigned long long> big(x->nsolve, 0x3ff0000000000000ULL); // 1.0 for every solve
     CK(cudaMemcpy2DAsync(&x->st.sc[0].sweep_max[slot - 1], sizeof(Scalars), big.data(), sizeof(unsigned long long),
                          sizeof(unsigned long long), x->nsolve, cudaMemcpyHostToDevice, x->stream));
-    auto launch = [&]() {
-        const SweepKernel k = sb == 64 ? sweep_kernel<MODEL, 64>(x, false, false)
-                              : sb == 256 ? sweep_kernel<MODEL, 256>(x, false, false) : sweep_kernel<MODEL, 128>(x, false, false);
-        k<<<x->gb_c * (BLOCK / sb), sb, 0, x->stream>>>(x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
-    };
-    launch();
+    const SweepKernel k = sb == 64    ? sweep_kernel<MODEL, 64>(x, false, false)
+                          : sb == 256 ? sweep_kernel<MODEL, 256>(x, false, false)
+                                      : sweep_kernel<MODEL, 128>(x, false, false);
+    const int grid = x->gb_c * (BLOCK / sb);
+    // the iteration's sweeps overlap the tail of the one before
+    x->chained = false;
+    launch(x, k, grid, sb, x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
     CK(cudaEventRecord(e0, x->stream));
-    for (int r = 0; r < reps; r++) launch();
+    for (int r = 0; r < reps; r++) launch(x, k, grid, sb, x->d_prm, x->mesh, x->st, slot, x->xcur, x->max_ni);
     CK(cudaEventRecord(e1, x->stream));
     CK(cudaGetLastError());
     CK(cudaMemset2DAsync(&x->st.sc[0].sweep_max[slot - 1], sizeof(Scalars), 0, 2 * sizeof(unsigned long long),

@@ -265,8 +265,8 @@ int csu_residual_norms_noalloc(const double* R, int nvar, int ncells, double* re
 
 /* Launch-shape autotuner (no counterpart in the reference): times the face-chunk size of the face-flux
  * kernel (32 or 64 faces per block reading their cells from global memory, or 128 faces per block staging
- * their cells through a shared-memory window) and the cell-block size of the DPLUR sweeps (64, 128 or 256) on this
- * context and keeps the fastest; neither choice changes a result bit. A context tunes itself on its first
+ * their cells through a shared-memory window) and the cell-block size of the DPLUR sweeps (64, 128 or 256; small
+ * meshes' sweeps run in 64 and are not timed) on this context and keeps the fastest; neither choice changes a result bit. A context tunes itself on its first
  * csu_iterate (16,384 cells or more; a cache per device, model and size class spares packs of a class seen
  * before the timing); this call re-times now and reports the choice. CSU_AUTOTUNE=0 in the environment
  * keeps the default shapes (64 faces, 128 cells). */
