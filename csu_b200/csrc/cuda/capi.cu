@@ -1899,7 +1899,7 @@ extern "C" int csu_dump(csu_ctx* x, int what, double* out)
         return CSU_OK;
     }
     case CSU_DUMP_SST_JAC: {
-        if (!x->st.dQ) {
+        if (!x->cfg.sst || !x->st.dQ) { // with saImplicitSource dQ holds SA's one row
             csu_set_error("csu_dump: no SST source Jacobians in this context (SST with LU-SGS or DPLUR only)");
             return CSU_ERR_STATE;
         }
