@@ -2037,7 +2037,8 @@ extern "C" int csu_prep_create(const csu_mesh_desc* md, const csu_config* cfg, c
         csu_set_error("csu_prep_create: mesh layout failed (a cell with more than four faces?)");
         return st;
     }
-    // device bytes of the solve: what a pack would carve for it alone, plus 1024 history rows
+    // device bytes of the solve: its share of a pack's arrays, cells padded to whole blocks and the solve maps of packs
+    // of several included (pack_build), plus 1024 history rows
     csu_ctx t;
     t.is_pack = true;
     t.pack_wall_d = p->L.wall_d != nullptr;
@@ -2045,8 +2046,11 @@ extern "C" int csu_prep_create(const csu_mesh_desc* md, const csu_config* cfg, c
     t.nv = nv;
     t.cfg = *cfg;
     t.L = p->L;
+    t.L.nc = (p->L.nc + BLOCK - 1) / BLOCK * BLOCK;
     Arena a;
     plan(&t, a);
+    carve<int>(a, t.L.nc / BLOCK);
+    carve<int>(a, t.L.nc);
     memset(&t.L, 0, sizeof(t.L)); // owned by p
     p->bytes = (long long)a.size + 1024LL * (nv + 4) * 8;
     *out = p;
