@@ -340,7 +340,7 @@ static int upload_mesh(csu_ctx* x)
     Mesh& m = x->mesh;
     auto up = [&](const void* dst, const void* src, size_t bytes) -> cudaError_t {
         if (bytes == 0) return cudaSuccess;
-        return cudaMemcpy(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice);
+        return cudaMemcpyAsync(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, x->stream);
     };
     std::vector<int2> fe(nf);
     std::vector<double2> fn(nf), fun(nf), r0(nf), r1(nf), bn(nb), fd(nf), bd(nb), bun(nb);
@@ -528,8 +528,7 @@ static int reset_scalars(csu_ctx* x, int it0)
         h.hist = hist_of(x, k);
         h.hist_cap = x->hist_cap;
     }
-    CK(cudaStreamSynchronize(x->stream));
-    CK(cudaMemcpy(x->st.sc, hs.data(), sizeof(Scalars) * hs.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(x->st.sc, hs.data(), sizeof(Scalars) * hs.size(), cudaMemcpyHostToDevice, x->stream));
     return CSU_OK;
 }
 
@@ -548,16 +547,14 @@ static int read_scalars(csu_ctx* x, Scalars* h)
 
 static int write_scalars_n(csu_ctx* x, const Scalars* h, int n)
 {
-    CK(cudaStreamSynchronize(x->stream));
-    CK(cudaMemcpy(x->st.sc, h, sizeof(Scalars) * n, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(x->st.sc, h, sizeof(Scalars) * n, cudaMemcpyHostToDevice, x->stream));
     return CSU_OK;
 }
 
 // host parameters to the device copy (after any change of prms)
 static int upload_prm(csu_ctx* x)
 {
-    CK(cudaStreamSynchronize(x->stream));
-    CK(cudaMemcpy(x->d_prm, x->prms.data(), sizeof(Prm) * x->nsolve, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(x->d_prm, x->prms.data(), sizeof(Prm) * x->nsolve, cudaMemcpyHostToDevice, x->stream));
     return CSU_OK;
 }
 
@@ -659,8 +656,10 @@ static int ctx_setup(csu_ctx* x)
     }
     x->arena.used = 0;
     plan(x, x->arena);
-    e = cudaMemset(x->arena.base, 0, bytes);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->own_stream, cudaStreamNonBlocking);
+    // The streams do not wait for the default one, so whatever a kernel reads is cleared and uploaded on the stream it runs
+    // on (a copy from pageable memory has left the caller's array when it returns, but may not have arrived).
+    e = cudaStreamCreateWithFlags(&x->own_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(x->arena.base, 0, bytes, x->own_stream);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x->ev_join, cudaEventDisableTiming);
@@ -2186,7 +2185,7 @@ extern "C" int csu_pack_transfer(csu_ctx* from, int kf, csu_ctx* to, int kt)
     ht.hist_row = 0;
     ht.steps = 0;
     ht.fresh = 0;
-    CK(cudaMemcpy(to->st.sc + kt, &ht, sizeof(Scalars), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(to->st.sc + kt, &ht, sizeof(Scalars), cudaMemcpyHostToDevice, to->stream));
     to->prepared = 0;
     return CSU_OK;
 }
@@ -2494,12 +2493,11 @@ static int seg_fill(csu_ctx* x, int k, const csu_layout* L, csu_ctx* src, int ks
         std::vector<std::vector<char>> keep;
         std::vector<const void*> from = seg_host(x->mesh, *L, keep);
         if (from.size() != dst.size()) return CSU_ERR_INPUT;
-        CK(cudaStreamSynchronize(x->stream));
         for (size_t a = 0; a < dst.size(); a++) {
             const size_t es = dst[a].es;
             const char* h = (const char*)from[a];
             auto up = [&](size_t so, size_t dof, size_t n) {
-                return cudaMemcpy(dst[a].dev + dof * es, h + so * es, n * es, cudaMemcpyHostToDevice);
+                return cudaMemcpyAsync(dst[a].dev + dof * es, h + so * es, n * es, cudaMemcpyHostToDevice, x->stream);
             };
             switch (dst[a].kind) {
             case SEG_CELL: CK(up(0, D.c0, D.nc)); break;
@@ -2628,14 +2626,14 @@ static int pack_build(const char* who, const csu_prep* const* solves, int n, csu
             for (int c = x->cell0[k]; c < c1; c++) cs[c] = k;
             for (int b = x->cell0[k] / BLOCK; b < (c1 + BLOCK - 1) / BLOCK; b++) bs[b] = k;
         }
-        cudaError_t e = cudaStreamSynchronize(x->stream);
-        if (e == cudaSuccess && n > 1) e = cudaMemcpy(const_cast<int*>(x->st.bsolve), bs.data(), sizeof(int) * nblk, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && n > 1) e = cudaMemcpy(const_cast<int*>(x->st.csolve), cs.data(), sizeof(int) * NC, cudaMemcpyHostToDevice);
-        for (int k = 0; k < n && e == cudaSuccess; k++)
-            e = cudaMemcpy(x->d_n2o + x->cell0[k], x->n2o[k].data(), sizeof(int) * x->ncs[k], cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && x->mesh.color_cells)
-            e = cudaMemcpy(const_cast<int*>(x->mesh.color_cells), color_cells.data(), sizeof(int) * NC,
-                           cudaMemcpyHostToDevice);
+        auto up = [&](const int* dst, const int* src, size_t count) {
+            return cudaMemcpyAsync(const_cast<int*>(dst), src, sizeof(int) * count, cudaMemcpyHostToDevice, x->stream);
+        };
+        cudaError_t e = cudaSuccess;
+        if (n > 1) e = up(x->st.bsolve, bs.data(), nblk);
+        if (e == cudaSuccess && n > 1) e = up(x->st.csolve, cs.data(), NC);
+        for (int k = 0; k < n && e == cudaSuccess; k++) e = up(x->d_n2o + x->cell0[k], x->n2o[k].data(), x->ncs[k]);
+        if (e == cudaSuccess && x->mesh.color_cells) e = up(x->mesh.color_cells, color_cells.data(), NC);
         if (e != cudaSuccess) st = cuda_fail(e, "pack maps");
     }
     if (!st) st = launch_lim3(x);
