@@ -9,7 +9,9 @@
 #include <algorithm>
 #include <mutex>
 #include <map>
+#include <memory>
 #include <tuple>
+#include <type_traits>
 #include "csu_gpu.h"
 #include "kernels.cuh"
 
@@ -1872,30 +1874,25 @@ extern "C" int csu_dump(csu_ctx* x, int what, double* out)
             csu_set_error("csu_dump: no DPLUR blocks in this context");
             return CSU_ERR_STATE;
         }
-        const size_t per = (size_t)nv * nv, ne = block_entries(x->model), slots = x->max_ni;
-        const size_t total = (size_t)(nc + 31) / 32 * 32 * slots * ne;
-        if (x->st.blocks) {
-            CK(d2h(a, x->st.blocks, total));
-        } else {
-            std::vector<float> f(total);
-            CK(cudaMemcpy(f.data(), x->st.blocks32, sizeof(float) * f.size(), cudaMemcpyDeviceToHost));
-            a.assign(f.begin(), f.end());
-        }
-        // entries that are always zero, and slots no cell has, are not stored
-        memset(out, 0, sizeof(double) * (size_t)nc * 4 * per);
-        for (int c = 0; c < nc; c++) {
-            double* o = out + (size_t)n2o[c] * 4 * per;
-            for (size_t j = 0; j < slots; j++) {
-                const double* e = a.data() + ((size_t)(c >> 5) * slots + j) * ne * 32 + (c & 31);
-                for (size_t q = 0; q < per; q++) {
-                    const int r = (int)(q / nv), k = (int)(q % nv);
-                    if (!block_nz(r, k)) continue;
-                    o[j * per + q] = *e;
-                    e += 32;
+        // entries that are always zero (at < 0 here), and slots no cell has, are not stored
+        const int per = nv * nv, ne = block_entries(x->model), slots = x->max_ni;
+        int at[36], stored = 0;
+        for (int q = 0; q < per; q++) at[q] = block_nz(q / nv, q % nv) ? 32 * stored++ : -1;
+        auto unpack = [&](const auto* dev) -> int {
+            using T = std::remove_cv_t<std::remove_pointer_t<decltype(dev)>>;
+            const size_t total = (size_t)(nc + 31) / 32 * 32 * slots * ne;
+            std::unique_ptr<T[]> host(new T[total]);
+            CK(cudaMemcpy(host.get(), dev, sizeof(T) * total, cudaMemcpyDeviceToHost));
+            for (int c = 0; c < nc; c++) {
+                double* o = out + (size_t)n2o[c] * 4 * per;
+                for (int j = 0; j < 4; j++, o += per) {
+                    const T* e = host.get() + ((size_t)(c >> 5) * slots + j) * ne * 32 + (c & 31);
+                    for (int q = 0; q < per; q++) o[q] = j < slots && at[q] >= 0 ? (double)e[at[q]] : 0.0;
                 }
             }
-        }
-        return CSU_OK;
+            return CSU_OK;
+        };
+        return x->st.blocks ? unpack(x->st.blocks) : unpack(x->st.blocks32);
     }
     case CSU_DUMP_SST_JAC: {
         if (!x->cfg.sst || !x->st.dQ) { // with saImplicitSource dQ holds SA's one row
