@@ -5,26 +5,25 @@
 // rounded to double. ext80.cuh reproduces that bit for bit with 128-bit integer arithmetic, which is exact
 // but costs ~1,000 integer instructions per gradient component.
 //
-// This header evaluates the same quantity in double-double arithmetic (FP64 pipes, error-free
-// transformations with explicit fma) together with a rigorous bound E on the distance between the
-// double-double value and the value the x87 sequence produces before its final rounding to double:
+// This header decides the same bits in FP64 (error-free transformations with explicit fma), in the two steps the
+// gradient kernel takes, with the integer model behind them:
 //
-//   - the sums A, B are reproduced exactly (x87_sum_add: each step rounded to 64 bits in FP64 with
-//     error-free transformations and an exact round-to-nearest-even on the 64-bit grid);
-//   - every later x87 operation rounds to a 64-bit significand, relative error <= u = 2^-64: the two
-//     products and the difference add u * |term| each, the division u * |q|;
-//   - the double-double evaluation itself is accurate to ~2^-100 relative (Joldes, Muller & Popescu,
-//     "Tight and rigorous error bounds for basic building blocks of double-word arithmetic", ACM TOMS
-//     2017), covered here by a 2^-96 term.
+//   - lsq_decide, for every component: the sums exactly, the quotient in double-double from constants already divided
+//     by the determinant, and a bound E on its distance from the value the x87 sequence has before its final rounding
+//     to double (every x87 operation rounds with relative error u = 2^-64; the double-double evaluation is accurate to
+//     about 2^-100, Joldes, Muller & Popescu, "Tight and rigorous error bounds for basic building blocks of
+//     double-word arithmetic", ACM TOMS 2017). If [q - E, q + E] rounds to one double, that is the x87 result. Open
+//     are 1 to 3 components in 100 of smooth fields, and about half of those of a field of one direction or on
+//     axis-aligned power-of-two spacings, where sums cancel or tie exactly.
+//   - for those, the x87 sums step by step (x87_sum2, x87_sum_add: each rounded to 64 bits with an exact
+//     round-to-nearest-even on that grid), the numerator exactly as x87 computes it, then the x87 division's rounding
+//     to 64 bits from the double-double quotient and its bound, and the store to double (lsq_exact_numerator). Open is
+//     a quotient within 2^-100 of a boundary of the 64-bit grid (none in millions of random components), or a
+//     magnitude outside the range the steps cover: ext80.cuh.
 //
-// If the interval [q - E, q + E] around the double-double value q contains no rounding boundary of
-// double precision (a midpoint between two consecutive doubles), the x87 result rounds to the same
-// double as q, namely RN(q): the component is certified and returned. Otherwise (about one component in
-// a hundred on solver meshes: strong cancellation in the numerator, or q close to a midpoint)
-// lsq_exact_numerator computes the numerator exactly as x87 would, then the x87 division's rounding to 64
-// bits from the double-double quotient and its bound, and the store to double exactly; what that cannot
-// decide (a quotient within 2^-100 of a boundary of the 64-bit grid: none in millions of random
-// components) the caller recomputes with ext80.cuh. Either way the result is the reference's bit pattern.
+// Either way the result is the reference's bit pattern. lsq_certified, between the two in cost, decides from the
+// rounded sums; the host check of the steps (tests/native/lsqdd_check.cpp) compares it too, the kernel
+// does not need it.
 #pragma once
 #include <math.h>
 #include <string.h>
@@ -104,22 +103,6 @@ X80_HD DD dd_mul(DD a, DD b)
     t = t + a.l * b.h;
     double c = p.l + t;
     return dd_fast_two_sum(p.h, c);
-}
-
-// An x87 value as an exact double-double (normal range only; m has bit 63 set or is zero).
-X80_HD DD dd_from_x80(X80 x)
-{
-    DD r;
-    if (x.m == 0) {
-        r.h = 0.0;
-        r.l = 0.0;
-        return r;
-    }
-    double hi = ldexp((double)(x.m >> 11), x.e + 11);
-    double lo = ldexp((double)(x.m & 0x7ffULL), x.e);
-    r = dd_fast_two_sum(hi, lo);
-    if (x.s) r = dd_neg(r);
-    return r;
 }
 
 // 1/d to ~2^-104 relative: one Newton correction of the FP64 reciprocal.
@@ -279,7 +262,7 @@ X80_HD bool lsq_certified(DD k1, DD k2, DD R, DD X, DD Y, double* out)
     return dd_round_certified(q, E, out);
 }
 
-// The same when lsq_certified cannot decide: the x87 numerator RN64(RN64(k1 X) - RN64(k2 Y)) computed
+// The same where the bound cannot decide: the x87 numerator RN64(RN64(k1 X) - RN64(k2 Y)) computed
 // exactly (x87_mul, x87_add), then the x87 division itself: RN64(N / det) decided on the 64-bit grid from
 // the double-double quotient N R (relative error <= 2^-103 (R) + 7 2^-106 (dd_mul) < 2^-102, bounded here by
 // 2^-100 |q|), and its store to double, RN53 of that 64-bit value, done exactly by the hardware addition in
@@ -311,7 +294,7 @@ X80_HD bool lsq_exact_numerator(DD k1, DD k2, DD R, DD X, DD Y, double* out)
 // The same decision without the intermediate 64-bit roundings, for the gradient kernel's every component: the
 // sums A = sum_j p_j exactly (as unevaluated h + l) instead of as x87 rounds them, the solve with the constants
 // already divided by the determinant, and every x87 rounding in the bound instead of in the arithmetic. About a
-// third of the operations of x87_sum_add and lsq_certified; undecided about as often (1 to 2 components in 100).
+// third of the operations of x87_sum_add and lsq_certified; undecided about as often.
 // ---------------------------------------------------------------------------------------------------------
 
 // Sum of products in the reference's order: h + l is the exact sum to 2^-104 b, b the sum of the |partial sums|,
