@@ -156,8 +156,8 @@ struct csu_ctx {
     bool tuned = false;      // launch shapes chosen (csu_autotune, or its cache on the first iteration)
     int device = 0;          // the CUDA device current when the context was made (its memory lives there)
     int sm_count = 148;      // that device's multiprocessors
-    // the renumbering on the device (packs: each solve's own), and for one-solve contexts a staging buffer for arrays in
-    // reference order (a pack stages one solve at a time in its face fluxes, which every iteration writes before it
+    // the renumbering on the device (packs: each solve's own), and for one-solve contexts a staging buffer for arrays
+    // in reference order (a pack stages one solve at a time in its face fluxes, which every iteration writes before it
     // reads them)
     int* d_n2o = nullptr;
     double* d_stage = nullptr;
@@ -658,8 +658,8 @@ static int ctx_setup(csu_ctx* x)
     }
     x->arena.used = 0;
     plan(x, x->arena);
-    // The streams do not wait for the default one, so whatever a kernel reads is cleared and uploaded on the stream it runs
-    // on (a copy from pageable memory has left the caller's array when it returns, but may not have arrived).
+    // The streams do not wait for the default one, so whatever a kernel reads is cleared and uploaded on the stream it
+    // runs on (a copy from pageable memory has left the caller's array when it returns, but may not have arrived).
     e = cudaStreamCreateWithFlags(&x->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMemsetAsync(x->arena.base, 0, bytes, x->own_stream);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x->side, cudaStreamNonBlocking);
@@ -781,10 +781,11 @@ extern "C" void csu_pack_arena_release(void)
     release_copy_jobs();
 }
 
-// The state of a solve between reference order ([var][cell], in the staging buffer) and the renumbered device layout (U4
-// + SoA scalars); k_state_in also marks the state as set from outside. Cells [c0, c0 + nc) of NC are solve k's (a
+// The state of a solve between reference order ([var][cell], in the staging buffer) and the renumbered device layout
+// (U4 + SoA scalars); k_state_in also marks the state as set from outside. Cells [c0, c0 + nc) of NC are solve k's (a
 // one-solve context: 0, all, 0). The renumbering was the host's for packs and residuals, most of their cost around few
-// iterations: 160,000-cell csu_residual 1.91 -> 1.01 ms, 8 SST solves set, 30 iterations and read back 19.5 -> 16.8 ms.
+// iterations: 160,000-cell csu_residual 1.91 -> 1.01 ms, 8 SST solves set, 30 iterations and read back
+// 19.5 -> 16.8 ms.
 __global__ void k_state_in(State s, const double* stage, const int* n2o, int nc, int nv, int c0, int NC, int k)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, c = c0 + i;
@@ -921,9 +922,10 @@ extern "C" int csu_get_state_rows(csu_ctx* x, double* const* U)
 // ---------------------------------------------------------------------------------------------- launches
 
 // A kernel of the iteration chain on the engine stream, allowed to start before the one launched just before it ends
-// (pdl_wait) when that was launched here too and nothing else came between: the launch itself and the loads of mesh rows
-// then overlap the previous kernel's tail. 3,049-cell RK5 7.85 -> 7.48 ms, LU-SGS wedge 3.46 -> 3.08 ms, a 5,000-cell
-// DPLUR solve with 20 sweeps 4.44 -> 3.82 ms, laminar request 5.56 -> 4.90 ms, 160,000-cell ramp 3.73 -> 3.51 ms.
+// (pdl_wait) when that was launched here too and nothing else came between: the launch itself and the loads of mesh
+// rows then overlap the previous kernel's tail. 3,049-cell RK5 7.85 -> 7.48 ms, LU-SGS wedge 3.46 -> 3.08 ms, a
+// 5,000-cell DPLUR solve with 20 sweeps 4.44 -> 3.82 ms, laminar request 5.56 -> 4.90 ms, 160,000-cell ramp
+// 3.73 -> 3.51 ms.
 template <typename... KA, typename... A>
 static void launch(csu_ctx* x, void (*k)(KA...), int grid, int block, A... args)
 {
@@ -1065,9 +1067,11 @@ static SweepKernel sweep_kernel_mode(const csu_ctx* x, bool first, bool last)
 {
     if (x->cfg.implicit_fp32)
         return first ? (last ? k_sweep<MODEL, true, true, SB, true, MODE> : k_sweep<MODEL, false, true, SB, true, MODE>)
-                     : (last ? k_sweep<MODEL, true, false, SB, true, MODE> : k_sweep<MODEL, false, false, SB, true, MODE>);
+                     : (last ? k_sweep<MODEL, true, false, SB, true, MODE>
+                             : k_sweep<MODEL, false, false, SB, true, MODE>);
     return first ? (last ? k_sweep<MODEL, true, true, SB, false, MODE> : k_sweep<MODEL, false, true, SB, false, MODE>)
-                 : (last ? k_sweep<MODEL, true, false, SB, false, MODE> : k_sweep<MODEL, false, false, SB, false, MODE>);
+                 : (last ? k_sweep<MODEL, true, false, SB, false, MODE>
+                         : k_sweep<MODEL, false, false, SB, false, MODE>);
 }
 
 // the sweep in blocks of SB cells
@@ -1075,7 +1079,8 @@ template <int MODEL, int SB>
 static SweepKernel sweep_kernel(const csu_ctx* x, bool first, bool last)
 {
     if constexpr (MODEL == 0) {
-        if (sweep_wide(MODEL, x->cfg.implicit_fp32, x->L.nc, x->sm_count)) return sweep_kernel_mode<MODEL, SB, SWEEP_WIDE>(x, first, last);
+        if (sweep_wide(MODEL, x->cfg.implicit_fp32, x->L.nc, x->sm_count))
+            return sweep_kernel_mode<MODEL, SB, SWEEP_WIDE>(x, first, last);
     }
     return sweep_kernel_mode<MODEL, SB, SWEEP_PLAIN>(x, first, last);
 }
@@ -1083,8 +1088,8 @@ static SweepKernel sweep_kernel(const csu_ctx* x, bool first, bool last)
 template <int MODEL, int SB>
 static void launch_sweep_sb(csu_ctx* x, int m, int n)
 {
-    launch(x, sweep_kernel<MODEL, SB>(x, m == 0, m == n - 1), x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur,
-           x->max_ni);
+    launch(x, sweep_kernel<MODEL, SB>(x, m == 0, m == n - 1), x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m,
+           x->xcur, x->max_ni);
 }
 
 template <int MODEL>
@@ -1092,9 +1097,13 @@ static void launch_sweep(csu_ctx* x, int m, int n)
 {
     if (m > 0 && early_sweeps(x)) {
         constexpr int M = MODEL < 2 ? MODEL : 0, SB = 64;
-        auto* k = x->cfg.implicit_fp32
-                      ? (m == n - 1 ? k_sweep<M, true, false, SB, true, SWEEP_EARLY> : k_sweep<M, false, false, SB, true, SWEEP_EARLY>)
-                      : (m == n - 1 ? k_sweep<M, true, false, SB, false, SWEEP_EARLY> : k_sweep<M, false, false, SB, false, SWEEP_EARLY>);
+        constexpr int E = SWEEP_EARLY;
+        const bool last = m == n - 1;
+        SweepKernel k;
+        if (x->cfg.implicit_fp32)
+            k = last ? k_sweep<M, true, false, SB, true, E> : k_sweep<M, false, false, SB, true, E>;
+        else
+            k = last ? k_sweep<M, true, false, SB, false, E> : k_sweep<M, false, false, SB, false, E>;
         launch(x, k, x->gb_c * (BLOCK / SB), SB, x->d_prm, x->mesh, x->st, m, x->xcur, x->max_ni);
         x->launches++;
         tmark(x, KSWEEP);
@@ -1143,7 +1152,8 @@ static void launch_iteration(csu_ctx* x)
             if (c.order == 2 || x->prm.visc) launch_grad<MODEL>(x, false);
             if (last) snapshot_views(x);
             launch_flux<MODEL>(x, last ? 1 : 0);
-            launch(x, last ? k_rk<MODEL, true> : k_rk<MODEL, false>, x->gb_c, BLOCK, x->d_prm, x->mesh, x->st, x->rk[sgi]);
+            launch(x, last ? k_rk<MODEL, true> : k_rk<MODEL, false>, x->gb_c, BLOCK, x->d_prm, x->mesh, x->st,
+                   x->rk[sgi]);
             x->launches++;
             tmark(x, KRK);
         }
@@ -1381,7 +1391,8 @@ static int time_flux_shape(csu_ctx* x, int fb, int reps, cudaEvent_t e0, cudaEve
     const int save = x->flux_fb;
     x->flux_fb = fb;
     const long long l0 = x->launches;
-    // as the iteration launches it: DPLUR's flux starts when the kernel before it has ended, the others' overlap its tail
+    // as the iteration launches it: DPLUR's flux starts when the kernel before it has ended, the others'
+    // overlap its tail
     x->chained = false;
     launch_flux<MODEL>(x, 1);
     CK(cudaEventRecord(e0, x->stream));
@@ -2221,8 +2232,8 @@ static std::vector<SegArr> seg_arrays(csu_ctx* x)
         {P(m.nei), 4, SEG_CELL4}, {P(m.lw), 16, SEG_CELL4}, {P(m.ld), 16, SEG_CELL4}, {P(m.lq), 16, SEG_CELL4},
         {P(m.lk), 16, SEG_CELL3}, {P(m.em), 16, SEG_CELL4}, {P(m.fslot), 4, SEG_CELL4}, {P(m.fnb), 4, SEG_CELL4},
         {P(m.omega), 8, SEG_CELL},
-        {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fun), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE}, {P(m.r0), 16, SEG_FACE},
-        {P(m.r1), 16, SEG_FACE}, {P(m.fd), 16, SEG_FACE}, {P(m.fL), 8, SEG_FACE},
+        {P(m.fe), 8, SEG_FACE}, {P(m.fn), 16, SEG_FACE}, {P(m.fun), 16, SEG_FACE}, {P(m.fds), 8, SEG_FACE},
+        {P(m.r0), 16, SEG_FACE}, {P(m.r1), 16, SEG_FACE}, {P(m.fd), 16, SEG_FACE}, {P(m.fL), 8, SEG_FACE},
         {P(m.bown), 4, SEG_BFACE}, {P(m.bflag), 4, SEG_BFACE}, {P(m.bold), 4, SEG_BFACE},
         {P(m.bn), 16, SEG_BFACE}, {P(m.bds), 8, SEG_BFACE}, {P(m.bd), 16, SEG_BFACE}, {P(m.bL), 8, SEG_BFACE},
         {P(m.bun), 16, SEG_BFACE}, {P(m.bds2), 8, SEG_BFACE}, {P(x->d_wall_rank), 4, SEG_BFACE}};

@@ -95,14 +95,15 @@ __global__ void __launch_bounds__(BLOCK) k_prim(const Prm* __restrict__ P, const
 // lsqdd.cuh, with the integer model only for the rare components those cannot decide.
 //
 // Bound by latency: a thread's chain of dependent FP64 operations and L2 loads. So a thread has one variable (four
-// lanes share a cell's double4 records), the certified solve keeps every x87 rounding in its bound instead of in
-// the arithmetic (lsq_decide), the two branches of the limiter are one, and the 1-3 % of components left undecided
-// are finished together, one per thread of the block. Against one thread per cell with the x87 sums emulated in
-// every component, the rare ones in a kernel behind it: 3,049 mixed cells 36.7 -> 16.7 us, 30,000
-// laminar 37.9 -> 22, 160,000 triangles 68 -> 59, 500,000 170 -> 147, the 209,825-quad SA plate 109 -> 100 (events, launch gap included; at
-// 160,000 triangles 8 % of the measured copy bandwidth for the 50 MB it must move). Measured and dropped: the
-// undecided components where they arise (67 us; a warp has one nearly every time), in a kernel of their own
-// (137 us at 500,000, but 28 us at 3,049), on a warp of their own beside the next group's (109 us).
+// lanes share a cell's double4 records), the certified solve keeps every x87 rounding in its bound instead of in the
+// arithmetic (lsq_decide), the two branches of the limiter are one, and the components left undecided (1-3 % of a
+// smooth field's, half of a one-directional one's) are finished together, one variable per thread of the block.
+// Against one thread per cell with the x87 sums emulated in every component, the rare ones in a kernel behind it:
+// 3,049 mixed cells 36.7 -> 16.7 us, 30,000 laminar 37.9 -> 22, 160,000 triangles 68 -> 58, 500,000 170 -> 138, the
+// 209,825-quad SA plate 109 -> 100 (events, launch gap included; at 160,000 triangles 13 % of the measured copy
+// bandwidth for the 50 MB it must move). Measured and dropped: the undecided components where they arise (67 us; a
+// warp has one nearly every time), in a kernel of their own (137 us at 500,000, but 28 us at 3,049), on a warp of
+// their own beside the next group's (109 us).
 // ------------------------------------------------------------------------------------------------
 constexpr int GRAD_CELLS = 32;
 
@@ -1139,9 +1140,9 @@ __global__ void __launch_bounds__(BLOCK) k_impl(const Prm* __restrict__ P, const
     if (WITH_R) partial_norms<MODEL>(s, valid, R);
 }
 
-// Step of the blocks' finite difference in variable mm (implicit.c:692). SST: rho omega reaches 1e10 beside a wall, where
-// a step of 1e-6 is below its last bit; its column (a flux linear in rho omega) and rho k's take a step relative to the
-// value.
+// Step of the blocks' finite difference in variable mm (implicit.c:692). SST: rho omega reaches 1e10 beside a wall,
+// where a step of 1e-6 is below its last bit; its column (a flux linear in rho omega) and rho k's take a step relative
+// to the value.
 constexpr double BLOCK_H = 1.0e-6;
 
 template <int MODEL>
@@ -1251,8 +1252,9 @@ __global__ void __launch_bounds__(BLOCK) k_side(const Prm* __restrict__ P, const
 // (43 -> 23). Registers for three blocks per SM (SST two; four: SA the same, 500,000 triangles 133).
 // ------------------------------------------------------------------------------------------------
 template <int MODEL>
-__global__ void __launch_bounds__(BLOCK, MODEL == 2 ? 2 : 3) k_blocks(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                                  const __grid_constant__ State s, int gb, int slots)
+__global__ void __launch_bounds__(BLOCK, MODEL == 2 ? 2 : 3)
+    k_blocks(const Prm* __restrict__ P, const __grid_constant__ Mesh m, const __grid_constant__ State s, int gb,
+             int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
     const int j = blockIdx.x / gb, cb = blockIdx.x - j * gb;
@@ -1366,17 +1368,26 @@ __device__ __forceinline__ void jacobi_update(const State& s, int nc, int c, dou
 // zeros in 32-cell tiles, each warp's a contiguous run (block_at): steady middle sweep of 160,000 triangles FP64
 // 16.5 -> 13.4 us, of 500,000 58 -> 47 us (244 MB, 5.2 TB/s, 79 % of the measured copy bandwidth), of the SA plate
 // (209,825 quads, FP32) 38.7 -> 23.8 us, SST airfoil pack 22 % faster per pass. SA's register budget is 96 (640
-// threads per SM): at the compiler's own 64 the plate's sweep takes 28.6 us, at 80 23.0 but the SA pack 5 % more;
-// Euler and SST are fastest at the compiler's choice (Euler held to 48: 16.7 us, SST held to 96 or 128: 2-5 % slower).
+// threads per SM in blocks of 64 and 128 cells; 128 in blocks of 256): at the compiler's own 64 the plate's sweep
+// takes 28.6 us, at 80 23.0 but the SA pack 5 % more; Euler and SST are fastest at the compiler's choice (Euler held
+// to 48: 16.7 us, SST held to 96 or 128: 2-5 % slower).
 //
 // On small meshes a sweep is one chain of loads: EARLY issues the gathers before the halt and early-exit flags arrive,
 // for registers that cost more than the chain once several waves hide it (sweep_early: where the line lies).
 //
 // WIDE holds Euler and laminar, 88 registers by themselves, to 56 in blocks of 64 and 128 cells and to 64 in blocks of
 // 256 (sweep_wide: on which meshes).
+// Blocks per SM of a sweep's register budget: WIDE 1,152 threads, SA 640, the others the compiler's choice.
+template <int MODEL, int SB, int MODE>
+constexpr int sweep_blocks()
+{
+    return MODE == SWEEP_WIDE ? 1152 / SB : MODEL == 1 && MODE == SWEEP_PLAIN ? 640 / SB : 1;
+}
+
 template <int MODEL, bool LAST, bool FIRST, int SB, bool F32, int MODE = SWEEP_PLAIN>
-__global__ void __launch_bounds__(SB, MODE == SWEEP_WIDE ? 1152 / SB : MODEL == 1 && MODE == SWEEP_PLAIN ? 640 / SB : 1) k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m,
-                                              const __grid_constant__ State s, int sweep, int cur, int slots)
+__global__ void __launch_bounds__(SB, sweep_blocks<MODEL, SB, MODE>())
+    k_sweep(const Prm* __restrict__ P, const __grid_constant__ Mesh m, const __grid_constant__ State s, int sweep,
+            int cur, int slots)
 {
     constexpr int NV = Model<MODEL>::NV, NP = Model<MODEL>::NP;
     constexpr bool EARLY = MODE == SWEEP_EARLY;
@@ -1388,7 +1399,7 @@ __global__ void __launch_bounds__(SB, MODE == SWEEP_WIDE ? 1152 / SB : MODEL == 
     int c = blockIdx.x * SB + threadIdx.x;
     const int nc = m.nc;
     const bool valid = cell_in(p, c);
-    // Slots 0-2 are gathered unconditionally (a slot without a face reads the cell itself and a zero block, both in
+    // Slots 0-2 are gathered unconditionally (a slot without a face reads the cell itself and some block, both in
     // bounds, and is not summed), so their index and neighbour loads issue together instead of one dependent chain
     // per face; slot 3 only exists in quadrilaterals. The indices are read before the wait for the previous sweep.
     int ni = 0, nbj[4] = {c, c, c, c};
@@ -1593,8 +1604,10 @@ __device__ __forceinline__ void delta_flux(const Prm& p, const double* P, const 
 //   FWD: x0_i = (-R_i - sum_{lower} 0.5 (dF(x0_j) dS - ra_j x0_j)) / D_i
 //   BWD: x1_i = (D_i x0_i - sum_{higher} 0.5 (dF(x1_j) dS - ra_j x1_j)) / D_i
 // A colour holds a quarter of the cells and depends on the one before, so a launch is one thread's latency, not
-// throughput: four lanes share a cell, one per face slot, and every lane then subtracts the faces' terms in slot order
-// (5,928-cell wedge: 12.5 -> 8.3 us a launch, 3 us of it the launch; the iteration 100 -> 65 us).
+// throughput: four lanes share a cell, one per face slot, and every lane then subtracts the faces' terms in slot order.
+// A launch between events, one lane -> four, meshes of 6,000, 100,000 and 300,000 cells: Euler 15.8 -> 8.3 us, 17.6 ->
+// 11.0, 22.1 -> 16.0; SST, whose lanes all repeat the diagonal block's x87 quotients, 19.1 -> 10.1, 22.3 -> 16.3, 31.5
+// -> 30.2 (5,928-cell wedge: the iteration 100 -> 57 us inside its graph).
 // ------------------------------------------------------------------------------------------------
 constexpr int LUSGS_THREADS = 128;
 

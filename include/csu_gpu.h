@@ -203,7 +203,8 @@ int csu_tube_run(csu_ctx* ctx, double tmax, int* steps, double* t_final);
  *  CSU_DUMP_BLOCKS  ncells*4*nvar*nvar          DPLUR blocks [cell][slot][row][col], slots in ELEMENT.f order
  *  CSU_DUMP_LSQ_X87 1                           gradient slots (cell, variable) so far that the FP64
  *                                               least squares could not decide and left to the integer x87
- *                                               model (no reference counterpart: a diagnostic of this engine)
+ *                                               model (none with CSU_LSQ=x87, which leaves nothing over; no
+ *                                               reference counterpart: a diagnostic of this engine)
  *  CSU_DUMP_SST_JAC 6*ncells                    SST source Jacobians dQkdr, dQkdrk, dQkdro, dQodr, dQodrk,
  *                                               dQodro [6][cell] of the last LU-SGS or DPLUR iteration
  *                                               (sst.c:643-680)
