@@ -1605,9 +1605,10 @@ __device__ __forceinline__ void delta_flux(const Prm& p, const double* P, const 
 //   BWD: x1_i = (D_i x0_i - sum_{higher} 0.5 (dF(x1_j) dS - ra_j x1_j)) / D_i
 // A colour holds a quarter of the cells and depends on the one before, so a launch is one thread's latency, not
 // throughput: four lanes share a cell, one per face slot, and every lane then subtracts the faces' terms in slot order.
-// A launch between events, one lane -> four, meshes of 6,000, 100,000 and 300,000 cells: Euler 15.8 -> 8.3 us, 17.6 ->
-// 11.0, 22.1 -> 16.0; SST, whose lanes all repeat the diagonal block's x87 quotients, 19.1 -> 10.1, 22.3 -> 16.3, 31.5
-// -> 30.2 (5,928-cell wedge: the iteration 100 -> 57 us inside its graph).
+// A launch between events, one lane -> four, meshes of 6,000, 100,000, 300,000 and 1,000,000 cells: Euler 15.8 -> 8.3
+// us, 17.6 -> 10.9, 22.1 -> 16.1, 55.8 -> 43.6; SST 19.1 -> 10.1, 22.3 -> 15.5, 31.5 -> 28.3, 78.2 -> 82.1 (its diagonal
+// block's x87 quotients one to a lane; repeated by every lane 87.3). 5,928-cell wedge: the iteration 100 -> 57 us in its
+// graph.
 // ------------------------------------------------------------------------------------------------
 constexpr int LUSGS_THREADS = 128;
 
@@ -1698,44 +1699,31 @@ __global__ void __launch_bounds__(LUSGS_THREADS) k_lusgs(const Prm* __restrict__
             const double v = __shfl_sync(0xffffffffu, term[k], q, 4);
             if (who >> q & 1u) x[k] -= v;
         }
+    // lane j finishes component j, lanes 0 and 1 a scalar each
+    double v = (j == 0 ? x[0] : j == 1 ? x[1] : j == 2 ? x[2] : x[3]) / D, vx = 0.0;
+    if constexpr (MODEL == 1) vx = x[4] / D;
     if constexpr (MODEL == 2) {
         // the SST diagonal (implicit.c:323-345, 444-465): D on the mean flow, a 2x2 block with the source
-        // Jacobians on k and omega, its determinant in double and the quotients in long double
-#pragma unroll
-        for (int k = 0; k < 4; k++) x[k] /= D;
-        const double A = x[4] + s.dQ[c] * x[0];
-        const double B = x[5] + s.dQ[(size_t)3 * nc + c] * x[0];
+        // Jacobians on k (lane 0) and omega (lane 1), its determinant in double and the quotients in long double
+        const double x0 = __shfl_sync(0xffffffffu, v, 0, 4);
+        const bool om = j & 1;
+        const double A = x[4] + s.dQ[c] * x0;
+        const double B = x[5] + s.dQ[(size_t)3 * nc + c] * x0;
         const double a = D - s.dQ[(size_t)nc + c], b = -s.dQ[(size_t)2 * nc + c];
         const double cq = -s.dQ[(size_t)4 * nc + c], dq = D - s.dQ[(size_t)5 * nc + c];
         const double det = a * dq - b * cq;
         if (fabs(det) < 1e-14) {
-            x[4] /= D;
-            x[5] /= D;
+            vx = (om ? x[5] : x[4]) / D;
         } else {
-            const double n4 = A * dq - B * b, n5 = -A * cq + B * a;
+            const double n = om ? -A * cq + B * a : A * dq - B * b;
             bool ok = true;
-            const double q4 = x87_div_d(n4, det, ok);
-            const double q5 = x87_div_d(n5, det, ok);
-            if (ok) {
-                x[4] = q4;
-                x[5] = q5;
-            } else {
-                const X80 dx = x80_from_double(det);
-                x[4] = x80_to_double(x80_div(x80_from_double(n4), dx));
-                x[5] = x80_to_double(x80_div(x80_from_double(n5), dx));
-            }
+            vx = x87_div_d(n, det, ok);
+            if (!ok) vx = x80_to_double(x80_div(x80_from_double(n), x80_from_double(det)));
         }
     }
     if (!store) return;
-    double4* dst4 = FWD ? s.X4[0] : s.X4[1];
-    double* dstx = FWD ? s.Xx[0] : s.Xx[1];
-    // lane j stores component j (and lane 0, 1 the scalars); without the SST block each divides its own
-    double v = j == 0 ? x[0] : j == 1 ? x[1] : j == 2 ? x[2] : x[3];
-    if constexpr (MODEL != 2) v /= D;
-    reinterpret_cast<double*>(dst4 + c)[j] = v;
-#pragma unroll
-    for (int k = 4; k < NV; k++)
-        if (j == k - 4) dstx[(size_t)(k - 4) * nc + c] = MODEL == 2 ? x[k] : x[k] / D;
+    reinterpret_cast<double*>((FWD ? s.X4[0] : s.X4[1]) + c)[j] = v;
+    if (j < NV - 4) (FWD ? s.Xx[0] : s.Xx[1])[(size_t)j * nc + c] = vx;
 }
 
 // U += dW1 (solverUpdateUImplicit), then the next iteration's primitives and clamps
