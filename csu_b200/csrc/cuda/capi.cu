@@ -951,10 +951,8 @@ static void launch_grad_lsq(csu_ctx* x)
     case 0: launch(x, k_grad<MODEL, DBG, 0>, g, t, x->d_prm, x->mesh, x->st); break;
     case 1: launch(x, k_grad<MODEL, DBG, 1>, g, t, x->d_prm, x->mesh, x->st); break;
     default:
-        // a mesh of at most three blocks per SM has no use for the register budget of more, whose spills its undecided
-        // components pay for (sod tube 90.4 -> 87.1 ms, 3,000-cell RK5 2.99 -> 2.89; beyond it the loads' latency
-        // shows: 20,000 cells laminar 3.46 ms by the larger budget's rule, SA 3.94, with this one 3.81 and 4.66)
-        if (!DBG && g <= 3 * x->sm_count) launch(x, k_grad<MODEL, false, 2, true>, g, t, x->d_prm, x->mesh, x->st);
+        if (!DBG && grad_small(MODEL, g, x->sm_count))
+            launch(x, k_grad<MODEL, false, 2, true>, g, t, x->d_prm, x->mesh, x->st);
         else launch(x, k_grad<MODEL, DBG, 2>, g, t, x->d_prm, x->mesh, x->st);
         break;
     }

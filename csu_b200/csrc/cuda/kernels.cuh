@@ -257,8 +257,8 @@ __device__ __forceinline__ void grad_finish(const Prm& p, const Mesh& m, const S
 
 // Blocks per SM of k_grad's register budget (64 registers; SST 72): with fewer the loads' latency shows (160,000
 // triangles, Euler: 4 blocks 68 us, 5 61, 6 59), with more the undecided components' code spills into the rest (8: 71).
-// SMALL: small meshes' undecided components without spills. LSQ 1: 80 registers (200,000 cells, RK5 with CSU_LSQ=x87:
-// 922 us an iteration; two blocks of 96 registers 1,025).
+// SMALL: small meshes' undecided components without spills (grad_small). LSQ 1: 80 registers (200,000 cells, RK5 with
+// CSU_LSQ=x87: 922 us an iteration; two blocks of 96 registers 1,025).
 template <int MODEL, int LSQ, bool SMALL>
 constexpr int grad_blocks()
 {
@@ -1606,9 +1606,9 @@ __device__ __forceinline__ void delta_flux(const Prm& p, const double* P, const 
 // A colour holds a quarter of the cells and depends on the one before, so a launch is one thread's latency, not
 // throughput: four lanes share a cell, one per face slot, and every lane then subtracts the faces' terms in slot order.
 // A launch between events, one lane -> four, meshes of 6,000, 100,000, 300,000 and 1,000,000 cells: Euler 15.8 -> 8.3
-// us, 17.6 -> 10.9, 22.1 -> 16.1, 55.8 -> 43.6; SST 19.1 -> 10.1, 22.3 -> 15.5, 31.5 -> 28.3, 78.2 -> 82.1 (its diagonal
-// block's x87 quotients one to a lane; repeated by every lane 87.3). 5,928-cell wedge: the iteration 100 -> 57 us in its
-// graph.
+// us, 17.6 -> 10.9, 22.1 -> 16.1, 55.8 -> 43.6; SST 19.1 -> 10.1, 22.3 -> 15.5, 31.5 -> 28.3, 78.2 -> 82.1 (its
+// diagonal block's x87 quotients one to a lane; repeated by every lane 87.3). 5,928-cell wedge: the iteration 100 -> 57
+// us in its graph.
 // ------------------------------------------------------------------------------------------------
 constexpr int LUSGS_THREADS = 128;
 

@@ -1,8 +1,21 @@
-// launch_rules.h -- which build of the DPLUR sweep a mesh gets, as functions of the mesh and the device alone.
+// launch_rules.h -- which build of the gradients and of the DPLUR sweep a mesh gets, as functions of the mesh and the
+// device alone.
 #pragma once
 #include <math.h>
 
 namespace csu {
+
+// Whether k_grad runs with the register budget of few blocks (SMALL): without the spills its undecided components pay
+// for, while the blocks an SM has fit in it. Per RK5 iteration on 148 multiprocessors, without -> with (cells, blocks an
+// SM):
+//   Euler    3,049 156.5 -> 151.2 us, 13,605 (2.9) 147.2 -> 141.1, 20,186 (4.3) 153.5 -> 166.8
+//   laminar  13,605 (2.9) 165.7 -> 157.6, 16,198 (3.4) 184.9 -> 202.6
+//   SA       9,120 (1.9) 195.3 -> 191.8, 12,182 (2.6) 198.7 -> 222.0
+//   SST      9,120 (1.9) 198.8 -> 194.7, 12,182 (2.6) 203.4 -> 228.2
+constexpr bool grad_small(int model, int blocks, int sms)
+{
+    return blocks <= (model == 0 ? 3 : 2) * sms;
+}
 
 // waves of `cells` cells on `sms` multiprocessors that hold `per_sm` of them at a time
 constexpr long long sweep_waves(long long cells, int per_sm, int sms)

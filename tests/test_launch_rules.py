@@ -40,7 +40,7 @@ def test_tune_class_separates_builds(rules):
     for fp32 in (0, 1):
         seen = {}
         sizes = range(16384, 700000, 97)
-        for cells, (wide, cls, early) in zip(sizes, rules([(0, fp32, c, 148) for c in sizes])):
+        for cells, (wide, cls, early, _) in zip(sizes, rules([(0, fp32, c, 148) for c in sizes])):
             assert seen.setdefault(cls, (wide, early)) == (wide, early), cells
         assert set(seen.values()) == {(0, 0), (0, 1), (1, 0)}
 
@@ -52,3 +52,11 @@ def test_early_by_cells_per_multiprocessor(rules, sms):
         at, above = rules([(model, fp32, per_sm * sms, sms), (model, fp32, per_sm * sms + 1, sms)])
         assert (at[2], above[2]) == (int(per_sm > 0), 0)
         assert not (at[0] or above[0])
+
+
+@pytest.mark.parametrize("sms", [148, 20])
+def test_small_gradient_budget_by_blocks_per_multiprocessor(rules, sms):
+    """Three blocks of 32 cells a multiprocessor for Euler and laminar, two for the wider blocks of SA and SST."""
+    for model, blocks in ((0, 3), (1, 2), (2, 2)):
+        at, above = rules([(model, 0, 32 * blocks * sms, sms), (model, 0, 32 * blocks * sms + 1, sms)])
+        assert (at[3], above[3]) == (1, 0)
