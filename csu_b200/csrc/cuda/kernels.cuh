@@ -99,11 +99,11 @@ __global__ void __launch_bounds__(BLOCK) k_prim(const Prm* __restrict__ P, const
 // arithmetic (lsq_decide), the two branches of the limiter are one, and the components left undecided (1-3 % of a
 // smooth field's, half of a one-directional one's) are finished together, one variable per thread of the block.
 // Against one thread per cell with the x87 sums emulated in every component, the rare ones in a kernel behind it:
-// 3,049 mixed cells 36.7 -> 16.7 us, 30,000 laminar 37.9 -> 22, 160,000 triangles 68 -> 58, 500,000 170 -> 138, the
-// 209,825-quad SA plate 109 -> 100 (events, launch gap included; at 160,000 triangles 13 % of the measured copy
-// bandwidth for the 50 MB it must move). Measured and dropped: the undecided components where they arise (67 us; a
-// warp has one nearly every time), in a kernel of their own (137 us at 500,000, but 28 us at 3,049), on a warp of
-// their own beside the next group's (109 us).
+// 3,049 mixed cells 36.7 -> 14.7 us, 30,000 laminar 37.9 -> 20.8, 160,000 triangles 68 -> 50, 500,000 170 -> 122, the
+// 209,825-quad SA plate 109 -> 94 (events, launch gap included; at 160,000 triangles 15 % of the measured copy
+// bandwidth for the 50 MB it must move). Measured and dropped, against an earlier 59 us at 160,000 and 147 at 500,000:
+// the undecided components where they arise (67 us; a warp has one nearly every time), in a kernel of their own (137 us
+// at 500,000, but 28 us at 3,049), on a warp of their own beside the next group's (109 us).
 // ------------------------------------------------------------------------------------------------
 constexpr int GRAD_CELLS = 32;
 

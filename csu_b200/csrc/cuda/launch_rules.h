@@ -6,8 +6,8 @@
 namespace csu {
 
 // Whether k_grad runs with the register budget of few blocks (SMALL): without the spills its undecided components pay
-// for, while the blocks an SM has fit in it. Per RK5 iteration on 148 multiprocessors, without -> with (cells, blocks an
-// SM):
+// for, while the blocks an SM has fit in it. Per RK5 iteration on 148 multiprocessors, without -> with (cells, blocks
+// an SM):
 //   Euler    3,049 156.5 -> 151.2 us, 13,605 (2.9) 147.2 -> 141.1, 20,186 (4.3) 153.5 -> 166.8
 //   laminar  13,605 (2.9) 165.7 -> 157.6, 16,198 (3.4) 184.9 -> 202.6
 //   SA       9,120 (1.9) 195.3 -> 191.8, 12,182 (2.6) 198.7 -> 222.0
